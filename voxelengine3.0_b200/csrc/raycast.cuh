@@ -16,19 +16,16 @@
 //
 //   A descent that restarts above level T0 reads one word of the scene's
 //   top table instead of levels 0..T0-1: per cell of the level-(T0-1)
-//   grid, the child-block offset reached at level T0, or the terminal level
-//   when the cell is empty higher up (built from the node words by
-//   k_build_top, bit-identical to walking them).  This shortens the longest
-//   descents of a warp — those that cross a coarse cell boundary — which set
-//   its lock-step cost.  Fetch-counting runs (COUNT) walk every level.
+//   grid, the child-block offset reached at level T0, or the size of the
+//   terminal cell when the walk ends higher up (built from the node words by
+//   k_build_top, bit-identical to walking them).  The grid has one layer of
+//   cells beyond 2^D on every axis, for the positions with a coordinate equal
+//   to 2^D that the bounds test admits.  Fetch-counting runs (COUNT) walk
+//   every level.
 //
 //   Where the table reaches the leaves (T0 = D, every scene of depth 3..10),
-//   a restart below level D is one table word and then the leaf word, so the
-//   only offset a ray keeps across steps is its leaf block's: the FLAT walk
-//   holds it in a register instead of the per-level array in local memory
-//   (trace 1.023 -> 0.998 ms, primary 0.398 -> 0.387 ms per 1080p depth-10
-//   frame).  Positions with a coordinate equal to 2^D, which the table does
-//   not cover, walk from the root.
+//   a restart below level D is one table word and then the leaf word: FlatRay
+//   and flat_step below, the walk of every frame kernel.
 #pragma once
 #include "ve_device.cuh"
 
@@ -58,7 +55,6 @@ struct Dda {
     float t_end;  // CLIP: past this distance the ray can hit nothing (set by the caller)
     uint32_t q, cc;
     uint32_t lux, luy, luz, e_last;
-    uint32_t bD;  // FLAT: offset of the leaf block (the child block reached at level D)
     uint32_t base[17];
 };
 
@@ -96,23 +92,21 @@ __device__ __forceinline__ bool dda_init(Dda& s, f3 o, f3 d, uint32_t controlche
     return false;
 }
 
+// Cells of the top table along an axis: 2^(T0-1) and the layer beyond 2^D.
+__host__ __device__ __forceinline__ uint32_t top_side(uint32_t T0) { return (1u << (T0 - 1u)) + 1u; }
 // Top-table entry of the cell containing (x, y, z): (offset << 1) | 1 when
 // levels 0..T0-1 are internal (offset = child block of the level-T0 node),
-// else (terminal level << 1).  The table covers positions below 2^D on every
-// axis (root child 0, which level 0's bit-D test selects for them).
+// else (size of the terminal cell - 1) << 1.
 __device__ __forceinline__ uint32_t top_index(uint32_t x, uint32_t y, uint32_t z, uint32_t D, uint32_t T0) {
-    const uint32_t sh = D - T0 + 1u, b = T0 - 1u;
-    return ((((x >> sh) << b) | (y >> sh)) << b) | (z >> sh);
+    const uint32_t sh = D - T0 + 1u, S = top_side(T0);
+    return ((x >> sh) * S + (y >> sh)) * S + (z >> sh);
 }
 
 // WORD: a hit reports the leaf's node word in h.id instead of its slot (the
 // bounce trace keeps the word for shading; the slot is the GBuffer's field).
 // CLIP: the ray also ends, as escaped, once its distance passes s.t_end —
 // for callers to whom an escape and a timeout are the same result.
-// FLAT: the scene's top table reaches the leaves (T0 = D): a descent is one
-// table word, then the leaf word, and the only offset kept across steps is
-// the leaf block's (a register, not the per-level array).
-template <bool COUNT, bool WORD = false, bool CLIP = false, bool FLAT = false>
+template <bool COUNT, bool WORD = false, bool CLIP = false>
 __device__ __forceinline__ bool dda_step(Dda& s, const uint32_t* __restrict__ nodes, uint64_t n_words, uint32_t D,
                                          const uint32_t* __restrict__ top, uint32_t T0, Hit& h, RayCount& rc) {
     const uint32_t L = 1u << D;
@@ -143,70 +137,20 @@ __device__ __forceinline__ bool dda_step(Dda& s, const uint32_t* __restrict__ no
         }
     }
     uint32_t k = s.e_last;
-    if (FLAT && !reuse) {
-        s.lux = ux; s.luy = uy; s.luz = uz;
-        bool found = false;
-        k = start;
-        const uint32_t sx = ux << 2, sy = uy << 1;
-        if (start < D) {
-            if (!((ux | uy | uz) & L)) {
-                const uint32_t ent = __ldg(top + top_index(ux, uy, uz, D, T0));
-                if (ent & 1u) {
-                    s.bD = ent >> 1;
-                    k = D;
-                } else {
-                    k = ent >> 1;
-                    found = true;
-                }
-            } else {
-                // a coordinate equal to 2^D (outside the table's cells): the
-                // walk from the root, reading the words the restart would
-                uint32_t b = 0u;
-                for (k = 0; k < D; k++) {
-                    const uint32_t sh = D - k;
-                    const uint32_t raw = fetch_node(nodes, n_words,
-                                                    b + (((sx >> sh) & 4u) | ((sy >> sh) & 2u) | ((uz >> sh) & 1u)));
-                    if (!(raw & 1u)) {
-                        found = true;
-                        break;
-                    }
-                    b = raw >> 4;
-                }
-                if (!found) s.bD = b;
-            }
-        }
-        s.e_last = k;
-        if (!found) {
-            const uint32_t off = s.bD + ((sx & 4u) | (sy & 2u) | (uz & 1u));
-            const uint32_t raw = fetch_node(nodes, n_words, off);
-            const uint32_t mat = (raw & 254u) >> 1;
-            if (mat != 0u) {
-                h.status = kHit;
-                h.id = WORD ? raw : off;
-                h.material = mat;
-                h.x = ux; h.y = uy; h.z = uz;
-                h.size = 1u;
-                h.checks = s.q;
-                return true;
-            }
-        }
-    } else if (!reuse) {
+    if (!reuse) {
         s.lux = ux; s.luy = uy; s.luz = uz;
         bool found = false;
         uint32_t off = 0;
         k = start;
         // child index at level k: bit D-k of x, y, z as bits 2, 1, 0
         const uint32_t sx = ux << 2, sy = uy << 1;
-        // inBounds admits a coordinate equal to 2^D; level 0 then selects
-        // another root child than the table's, so such a position walks
-        // every level as the reference's descent does
-        if (!COUNT && start < T0 && !((ux | uy | uz) & L)) {
+        if (!COUNT && start < T0) {
             const uint32_t ent = __ldg(top + top_index(ux, uy, uz, D, T0));
             if (ent & 1u) {
                 s.base[T0] = ent >> 1;
                 k = T0;
             } else {
-                k = ent >> 1;
+                k = D - uint32_t(__popc(ent >> 1));  // cell size 2^(D-k)
                 found = true;
             }
         }
@@ -255,19 +199,161 @@ __device__ __forceinline__ bool dda_step(Dda& s, const uint32_t* __restrict__ no
     return false;
 }
 
+// ---------------------------------------------------------------------------
+// The walk of scenes whose top table reaches the leaves (T0 = D).
+//
+// Bound by issue: a step is arithmetic between two dependent loads, so it is
+// written for few instructions.  With the result stores moved to the refill
+// (k_trace) it took the trace of a 1080p depth-10 frame (4 spp x 3 bounces)
+// from 0.963 to 0.694 ms (155.9 M -> 88.2 M warp instructions in the first
+// pass of its 960x540 form) and the primary pass from 0.382 to 0.346 ms.
+//   * Positions are kept as the bits of r + 1.5 * 2^23 rounded toward zero
+//     (r in [0, 2^16]: the low 22 bits are trunc(r) exactly), one full-rate
+//     add in place of a quarter-rate conversion, and the far plane of a cell
+//     goes back to a float by subtracting that constant (exact).  The plane
+//     itself is one logic operation: with c = the bits of -1.5 * 2^23 + 1 for
+//     a rising axis (low 22 bits all ones) and of -1.5 * 2^23 for a falling one
+//     (all zeros), ((b ^ c) & ~m) ^ c is the cell's last coordinate or its
+//     first one (m = cell size - 1), and adding c as a float gives the plane.
+//   * The cell is one mask m, compared with the changed bits of the position:
+//     no level, no leading-zero count.
+//   * min/max of three operands are one instruction each.  They return what
+//     the glm selects of dda_step return: inside the volume no exit distance
+//     is NaN (an axis with 1/d = +-inf has a non-zero numerator of its sign),
+//     and the bounds test propagates NaN to "outside" as the comparisons do.
+//   * The table's index arithmetic runs on the biased bits; the table pointer
+//     takes the bias out once per ray (flat_top).
+// Table entries below 2^31 and blocks at most n_words (k_build_top clamps; the
+// node array ends with 8 zero words) make both loads unconditional.
+// ---------------------------------------------------------------------------
+constexpr float kPosBias = 12582912.0f;         // 1.5 * 2^23
+constexpr uint32_t kPosBits = 0x4B400000u;      // its bits
+constexpr uint32_t kPlaneRise = 0xCB3FFFFFu;    // bits of 1 - 1.5 * 2^23
+enum : uint32_t { kWalking = 3u };              // flat_step: the ray goes on
+
+struct FlatRay {
+    f3 o, d, inv;
+    float t, t_end;
+    uint32_t left;        // steps before the timeout
+    uint32_t bx, by, bz;  // biased position bits of the last step
+    uint32_t m;           // size - 1 of its cell
+    uint32_t blk;         // m = 0: its leaf block; after a hit: the leaf's word (WORD) or slot
+};
+
+// Table pointer such that the index of the biased bits, modulo 2^32, lands on
+// the cell: index + K with K = (kPosBits >> 1) * (S^2 + S + 1) mod 2^32 does
+// not wrap for any table (S = 2^2 + 1 .. 2^9 + 1).
+__device__ __forceinline__ const uint32_t* flat_top(const uint32_t* top, uint32_t S) {
+    const uint32_t K = (kPosBits >> 1) * (S * S + S + 1u);
+    return reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(top) - 4ull * K);
+}
+__device__ __forceinline__ float min3_nan(float a, float b, float c) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// Distance to the far plane of the cell along one axis.
+__device__ __forceinline__ float flat_exit(uint32_t b, uint32_t m, float o, float inv) {
+    const uint32_t neg = __float_as_uint(inv) >> 31;
+    const uint32_t c = kPlaneRise + neg;
+    const float plane = __uint_as_float(((b ^ c) & ~m) ^ c) + __uint_as_float(c);
+    const float e = __uint_as_float((__float_as_uint(inv) & 0x80000000u) | __float_as_uint(0.001f));
+    return ((plane - o) + e) * inv;
+}
+
+// Returns false when the ray misses the volume (escaped; `left` is then one
+// less than the checks allow).
+__device__ __forceinline__ bool flat_init(FlatRay& s, f3 o, f3 d, uint32_t controlchecks, float Lf) {
+    s.inv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+    s.d = d;
+    s.o = add(o, muls(d, 4.0f));
+    s.left = controlchecks + 1u;
+    s.bx = s.by = s.bz = 0u;  // no position yet: every bit differs from the first step's
+    s.m = 0u;
+    s.blk = 0u;
+    s.t = 0.0f;
+    if (!in_bounds(s.o, Lf)) {
+        const f3 t1 = mul(mk((0.0f - s.o.x) + 0.001f, (0.0f - s.o.y) + 0.001f, (0.0f - s.o.z) + 0.001f), s.inv);
+        const f3 t2 = mul(mk((Lf - s.o.x) - 0.001f, (Lf - s.o.y) - 0.001f, (Lf - s.o.z) - 0.001f), s.inv);
+        const float t_enter = gmax(gmax(gmin(t1.x, t2.x), gmin(t1.y, t2.y)), gmin(t1.z, t2.z));
+        const float t_exit = gmin(gmin(gmax(t1.x, t2.x), gmax(t1.y, t2.y)), gmax(t1.z, t2.z));
+        s.left--;
+        if (t_exit < t_enter || t_exit < 0.0f) return false;
+        s.t = t_enter;
+    }
+    return true;
+}
+
+// One iteration of the reference loop: kWalking, or how the ray ended (kHit /
+// kEscaped / kTimeout).  WORD: a hit leaves the leaf's word in blk, else its
+// slot.  CLIP as in dda_step.
+template <bool WORD, bool CLIP>
+__device__ __forceinline__ uint32_t flat_step(FlatRay& s, const uint32_t* __restrict__ nodes,
+                                              const uint32_t* __restrict__ topb, uint32_t S, float Lf) {
+    const f3 r = add(muls(s.d, s.t), s.o);
+    const float lo = min3_nan(r.x, r.y, r.z), hi = max3_nan(r.x, r.y, r.z);
+    if (!(0.0f <= lo && hi <= Lf) || (CLIP && s.t > s.t_end)) return kEscaped;
+    if (s.left == 0u) return kTimeout;
+    s.left--;
+    const uint32_t bx = __float_as_uint(__fadd_rz(r.x, kPosBias));
+    const uint32_t by = __float_as_uint(__fadd_rz(r.y, kPosBias));
+    const uint32_t bz = __float_as_uint(__fadd_rz(r.z, kPosBias));
+    const uint32_t xd = (bx ^ s.bx) | (by ^ s.by) | (bz ^ s.bz);
+    s.bx = bx; s.by = by; s.bz = bz;
+    if (xd > s.m) {            // another cell
+        if (xd > (s.m | 1u)) {  // ... and not of the same leaf block
+            const uint32_t ent = __ldg(topb + (((bx >> 1) * S + (by >> 1)) * S + (bz >> 1)));
+            s.m = (ent & 1u) ? 0u : ent >> 1;
+            s.blk = ent >> 1;
+        }
+        if (s.m == 0u) {
+            const uint32_t off = s.blk + (((bx << 2) & 4u) | ((by << 1) & 2u) | (bz & 1u));
+            const uint32_t raw = __ldg(nodes + off);
+            if (raw & 254u) {
+                s.blk = WORD ? raw : off;
+                return kHit;
+            }
+        }
+    }
+    s.t = fminf(fminf(flat_exit(bx, s.m, s.o.x, s.inv.x), flat_exit(by, s.m, s.o.y, s.inv.y)),
+                flat_exit(bz, s.m, s.o.z, s.inv.z));
+    return kWalking;
+}
+
 template <bool COUNT>
 __device__ __forceinline__ Hit raycast(const uint32_t* __restrict__ nodes, uint64_t n_words, uint32_t D,
                                        const uint32_t* __restrict__ top, uint32_t T0, f3 o, f3 d,
                                        uint32_t controlchecks, RayCount& rc) {
-    Dda s;
     Hit h;
-    if (dda_init(s, o, d, controlchecks, D, h)) return h;
     if (!COUNT && T0 == D) {
-        while (!dda_step<COUNT, false, false, true>(s, nodes, n_words, D, top, T0, h, rc)) {
+        const uint32_t S = top_side(T0);
+        const float Lf = float(1u << D);
+        const uint32_t* topb = flat_top(top, S);
+        FlatRay s;
+        h.status = kEscaped;
+        h.id = h.material = h.x = h.y = h.z = h.size = 0;
+        if (flat_init(s, o, d, controlchecks, Lf)) {
+            do h.status = flat_step<false, false>(s, nodes, topb, S, Lf);
+            while (h.status == kWalking);
         }
-    } else {
-        while (!dda_step<COUNT>(s, nodes, n_words, D, top, T0, h, rc)) {
+        // the reference's count includes the check that found no steps left
+        h.checks = controlchecks + 1u - s.left + (h.status == kTimeout ? 1u : 0u);
+        if (h.status == kHit) {
+            h.id = s.blk;
+            h.material = (__ldg(nodes + s.blk) & 254u) >> 1;
+            h.x = s.bx - kPosBits; h.y = s.by - kPosBits; h.z = s.bz - kPosBits;
+            h.size = 1u;
         }
+        return h;
+    }
+    Dda s;
+    if (dda_init(s, o, d, controlchecks, D, h)) return h;
+    while (!dda_step<COUNT>(s, nodes, n_words, D, top, T0, h, rc)) {
     }
     return h;
 }

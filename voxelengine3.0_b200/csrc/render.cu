@@ -58,7 +58,7 @@ struct DevScene {
     uint32_t cache_log2;
     uint32_t probes;
     uint32_t top_level;   // T0: levels 0..T0-1 resolved by the top table (0: none)
-    const uint32_t* top;  // top table, (2^(T0-1))^3 words
+    const uint32_t* top;  // top table, top_side(T0)^3 words
     // emissive lights (VE_FRAME_EMISSIVE; null until the scene's first such frame)
     EmLight* em_list;     // the registry, kEmCapacity records
     uint32_t* em_claim;   // claim table of registered (or dropped) light vids
@@ -413,89 +413,45 @@ __global__ void __launch_bounds__(256) k_decay(CacheEntry* cache, uint32_t n, fl
 
 // trace.comp:25-70 for extension rays; shadow rays test escape toward the sun.
 //
-// Persistent kernel with per-lane refill: a lane whose ray has finished takes
-// the next queue entry (one warp-aggregated atomicAdd on a per-pass cursor
-// serves all idle lanes of the warp, once `refill` of them are idle or none is
-// busy), so warps stay full although ray lengths differ by 100x.  One ballot
-// per step: once a refill hands out the queue's last entry the warp stops
-// refilling (a warp-uniform flag) and runs its remaining rays out.
+// Persistent kernel with per-lane refill: lanes whose rays have finished keep
+// the result in registers until `refill` of them are idle (or none is busy);
+// then all of them store their results and take the next queue entries at
+// once (one warp-aggregated atomicAdd on a per-pass cursor), so warps stay
+// full although ray lengths differ by 100x, and the code around a step runs
+// for many lanes at a time: about 2 rays of a warp end per step, and storing
+// each result where it ended cost as much as a third of the step.  Once a
+// refill hands out the queue's last entry the warp stops refilling (a
+// warp-uniform flag) and runs its remaining rays out.
 // EM: the batch has VE_FRAME_EMISSIVE views (shadow rays toward lights).
-// FLAT: every scene of the batch has a top table reaching its leaves
-// (T0 = D): the descent keeps one leaf-block offset instead of the per-level
-// array (dda_step).
+// FLAT: every scene of the batch has a top table reaching its leaves (T0 = D):
+// flat_step.  Fetch-counting batches take the general walk.
+enum : uint32_t { kLaneIdle = 4u };  // lane state: kWalking, a finished ray's status to be stored, or no ray
 template <bool COUNT, bool EM = false, bool FLAT = false>
 __global__ void __launch_bounds__(256, 6) k_trace(FrameArgs a, uint32_t pass) {
+    static_assert(!(COUNT && FLAT), "fetch counts need the walk of every level");
     // the pass's extension rays, then its shadow rays: warps stay mostly of
     // one kind, and the shorter shadow rays form the tail of the pass
     const uint32_t n_ext = a.counters[CNT_RAY + pass];
     const uint32_t n = n_ext + a.counters[CNT_RAYSH + pass];
     uint32_t* cursor = &a.counters[CNT_CURSOR + pass];
     const uint32_t lane = lane_id();
-    bool active = false;
     bool drained = false;  // warp-uniform: every ray of the pass has been handed out
+    uint32_t state = kLaneIdle;
     uint32_t e = 0, D = 0, T0 = 0;
     const uint32_t* nodes = nullptr;
     const uint32_t* top = nullptr;
     uint32_t n_words = 0;
+    float Lf = 0.0f;  // FLAT: 2^D, and the table's side in T0
     Dda s;
+    FlatRay fr;
+    Hit h;
     RayCount rc;
     for (;;) {
-        // the result lives one iteration: written and stored when a ray ends
-        Hit h;
-        h.status = kEscaped;
-        h.id = h.material = h.x = h.y = h.z = 0u;
-        const unsigned busy = __ballot_sync(0xffffffffu, active);
-        if (drained && busy == 0u) break;
-        const unsigned idle = drained ? 0u : ~busy;
-        bool finished = false;
-        if (idle != 0u && (uint32_t(__popc(idle)) >= a.refill || busy == 0u)) {
-            const int leader = __ffs(idle) - 1;
-            uint32_t first_idx = 0;
-            if (int(lane) == leader) first_idx = atomicAdd(cursor, uint32_t(__popc(idle)));
-            first_idx = __shfl_sync(0xffffffffu, first_idx, leader);
-            drained = first_idx + uint32_t(__popc(idle)) >= n;
-            if (!active) {
-                const uint32_t idx = first_idx + uint32_t(__popc(idle & ((1u << lane) - 1u)));
-                if (idx < n) {
-                    const uint2 en = idx < n_ext ? a.rayq[idx] : a.rayq_sh[idx - n_ext];
-                    e = en.x;
-                    const uint32_t p = e & 0x3FFFFFFFu;
-                    const DevView& v = a.views[en.y];
-                    const DevScene S = a.scenes[v.scene];
-                    nodes = S.nodes;
-                    n_words = word_bound(S.n_words);
-                    D = S.depth;
-                    top = S.top;
-                    T0 = S.top_level;
-                    const f3 o = ld3(a.p_ray_o[p]);
-                    f3 d = (e >> 31) ? mk(v.sun[0], v.sun[1], v.sun[2]) : ld3(a.p_ray_d[p]);
-                    if (EM && (e >> 31) && (v.flags & VE_FRAME_EMISSIVE)) d = ld3(a.p_sdir[p]);
-                    finished = dda_init(s, o, d, v.cc_bounce, D, h);
-                    {
-                        // a bounce ray that escapes or times out shades as
-                        // sky alike, so it ends on leaving the box of the
-                        // cells that can hold a voxel (exit of its slab);
-                        // shadow rays walk on (there a timeout is a shadow).
-                        // Fetch-counting frames count this walk too.
-                        float te = __int_as_float(0x7f800000);
-                        if (!(e >> 31)) {
-                            const float tx = ((s.inv.x > 0.0f ? S.clip_hi[0] : S.clip_lo[0]) - s.o.x) * s.inv.x;
-                            const float ty = ((s.inv.y > 0.0f ? S.clip_hi[1] : S.clip_lo[1]) - s.o.y) * s.inv.y;
-                            const float tz = ((s.inv.z > 0.0f ? S.clip_hi[2] : S.clip_lo[2]) - s.o.z) * s.inv.z;
-                            te = gmin(gmin(tx, ty), tz);
-                        }
-                        s.t_end = te;
-                    }
-                    active = !finished;
-                }
-            }
-        }
-        if (active) {
-            finished = dda_step<COUNT, true, true, FLAT && !COUNT>(s, nodes, n_words, D, top, T0, h, rc);
-            if (finished) active = false;
-        }
-        if (finished) {
+        if (state < kWalking) {  // store a finished ray's result
             const uint32_t p = e & 0x3FFFFFFFu;
+            const uint32_t word = FLAT ? fr.blk : h.id;
+            const uint32_t x = FLAT ? fr.bx - kPosBits : h.x, y = FLAT ? fr.by - kPosBits : h.y,
+                           z = FLAT ? fr.bz - kPosBits : h.z;
             if (e >> 31) {
                 // the shadow ray's result code: ~0 left the volume, a hit
                 // voxel's vid (emissive batches: the light must be the hit),
@@ -505,17 +461,77 @@ __global__ void __launch_bounds__(256, 6) k_trace(FrameArgs a, uint32_t pass) {
                 // take the same code.
                 uint32_t* rec = reinterpret_cast<uint32_t*>(a.p_pend + p) + 3;
                 if (!EM && (e & 0x40000000u)) {
-                    const uint32_t n = *rec, code = h.status == kEscaped ? 0xFFFFFFFFu : 0u;
-                    for (uint32_t k = 0; k <= n; k++) rec[4u * k] = code;
-                } else if (h.status == kEscaped) {
+                    const uint32_t cnt = *rec, code = state == kEscaped ? 0xFFFFFFFFu : 0u;
+                    for (uint32_t k = 0; k <= cnt; k++) rec[4u * k] = code;
+                } else if (state == kEscaped) {
                     *rec = 0xFFFFFFFFu;
-                } else if (EM && h.status == kHit) {
-                    *rec = voxel_key(h.x, h.y, h.z) + 1u;
+                } else if (EM && state == kHit) {
+                    *rec = voxel_key(x, y, z) + 1u;
                 }
             } else {
-                // h.id holds the hit leaf's word: the shade pass needs no
-                // dependent load from the node array
-                a.p_hit[p] = make_uint4(h.status, h.id, h.x | (h.y << 16), h.z | (h.material << 16));
+                // the hit leaf's word rides along: the shade pass needs no
+                // dependent load from the node array.  It reads the rest of
+                // the record for a hit only.
+                a.p_hit[p] = make_uint4(state, word, x | (y << 16), z | (((word & 254u) >> 1) << 16));
+            }
+            state = kLaneIdle;
+        }
+        if (drained) break;  // the last rays have just been stored
+        const unsigned idle = __ballot_sync(0xffffffffu, state == kLaneIdle);
+        const uint32_t want = uint32_t(__popc(idle));
+        const int leader = __ffs(idle) - 1;
+        uint32_t first_idx = 0;
+        if (int(lane) == leader) first_idx = atomicAdd(cursor, want);
+        first_idx = __shfl_sync(0xffffffffu, first_idx, leader);
+        drained = first_idx + want >= n;
+        if (state == kLaneIdle) {
+            const uint32_t idx = first_idx + uint32_t(__popc(idle & ((1u << lane) - 1u)));
+            if (idx < n) {
+                const uint2 en = idx < n_ext ? a.rayq[idx] : a.rayq_sh[idx - n_ext];
+                e = en.x;
+                const uint32_t p = e & 0x3FFFFFFFu;
+                const DevView& v = a.views[en.y];
+                const DevScene& S = a.scenes[v.scene];
+                nodes = S.nodes;
+                const f3 o = ld3(a.p_ray_o[p]);
+                f3 d = (e >> 31) ? mk(v.sun[0], v.sun[1], v.sun[2]) : ld3(a.p_ray_d[p]);
+                if (EM && (e >> 31) && (v.flags & VE_FRAME_EMISSIVE)) d = ld3(a.p_sdir[p]);
+                bool go;
+                if (FLAT) {
+                    T0 = top_side(S.top_level);
+                    top = flat_top(S.top, T0);
+                    Lf = float(1u << S.depth);
+                    go = flat_init(fr, o, d, v.cc_bounce, Lf);
+                } else {
+                    n_words = word_bound(S.n_words);
+                    D = S.depth;
+                    top = S.top;
+                    T0 = S.top_level;
+                    go = !dda_init(s, o, d, v.cc_bounce, D, h);
+                }
+                state = go ? kWalking : kEscaped;
+                // a bounce ray that escapes or times out shades as sky alike,
+                // so it ends on leaving the box of the cells that can hold a
+                // voxel (exit of its slab); shadow rays walk on (there a
+                // timeout is a shadow).  Fetch-counting frames count this
+                // walk too.
+                const f3 ro = FLAT ? fr.o : s.o, ri = FLAT ? fr.inv : s.inv;
+                float te = __int_as_float(0x7f800000);
+                if (!(e >> 31)) {
+                    const float tx = ((ri.x > 0.0f ? S.clip_hi[0] : S.clip_lo[0]) - ro.x) * ri.x;
+                    const float ty = ((ri.y > 0.0f ? S.clip_hi[1] : S.clip_lo[1]) - ro.y) * ri.y;
+                    const float tz = ((ri.z > 0.0f ? S.clip_hi[2] : S.clip_lo[2]) - ro.z) * ri.z;
+                    te = gmin(gmin(tx, ty), tz);
+                }
+                fr.t_end = s.t_end = te;
+            }
+        }
+        // step until `refill` lanes are idle; run all out once drained
+        const int lim = drained ? 0 : 32 - int(a.refill);
+        while (__popc(__ballot_sync(0xffffffffu, state == kWalking)) > lim) {
+            if (state == kWalking) {
+                if (FLAT) state = flat_step<true, true>(fr, nodes, top, T0, Lf);
+                else if (dda_step<COUNT, true, true>(s, nodes, n_words, D, top, T0, h, rc)) state = h.status;
             }
         }
     }
@@ -1988,6 +2004,11 @@ static int fail(int code, const std::string& msg) {
             return fail(VE_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));               \
     } while (0)
 
+// words of a node array's allocation besides its own: 7 in front (every
+// 8-child block starts on a 32-byte boundary) and 8 zero words behind it (the
+// block that top-table entries past the end point at), rounded up
+constexpr size_t kNodePad = 16;
+
 struct SceneSlot {
     void* alloc = nullptr;   // node array allocation (nodes start 7 words in)
     uint32_t* nodes = nullptr;
@@ -2220,31 +2241,32 @@ static int sync_scenes(ve_ctx* c) {
 // level D steps over an empty cell (only level-D words are tested for a
 // material), so only cells internal down to level T0 can be hit.  box[0..2]
 // = smallest, box[3..5] = largest such cell coordinate (box[0] > box[3]: no
-// such cell).  Positions with a coordinate equal to 2^D lie outside the
-// table; k_face_hits covers them.
+// such cell).  Positions with a coordinate equal to 2^D (the last layer of
+// cells on each axis) are left out of the box; k_face_hits covers them.
 __global__ void k_build_top(const uint32_t* __restrict__ nodes, uint64_t n_words, uint32_t D, uint32_t T0,
                             uint32_t* __restrict__ top, uint32_t* __restrict__ box) {
     __shared__ uint32_t sb[6];
     if (threadIdx.x < 6) sb[threadIdx.x] = threadIdx.x < 3 ? 0xFFFFFFFFu : 0u;
-    const uint32_t b = T0 - 1u, n = 1u << (3u * b);
+    const uint32_t side = top_side(T0), n = side * side * side;
     const uint32_t sh = D - T0 + 1u, L = 1u << D;
     uint32_t lo[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, hi[3] = {0u, 0u, 0u};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t cx = i >> (2u * b), cy = (i >> b) & ((1u << b) - 1u), cz = i & ((1u << b) - 1u);
+        const uint32_t cz = i % side, cy = (i / side) % side, cx = i / (side * side);
         const uint32_t x = cx << sh, y = cy << sh, z = cz << sh;
         uint32_t base = 0, ent = 0;
         bool terminal = false;
         for (uint32_t k = 0; k < T0; k++) {
             const uint32_t raw = dev::fetch_node(nodes, n_words, base + locate(x, y, z, L >> k));
             if (!(raw & 1u)) {
-                ent = k << 1;
+                ent = ((L >> k) - 1u) << 1;
                 terminal = true;
                 break;
             }
             base = raw >> 4;
         }
-        top[i] = terminal ? ent : ((base << 1) | 1u);
-        if (!terminal) {
+        // a block past the end reads as the zero words that follow the array
+        top[i] = terminal ? ent : ((min(base, uint32_t(n_words)) << 1) | 1u);
+        if (!terminal && max(max(cx, cy), cz) + 1u < side) {
             lo[0] = min(lo[0], cx); lo[1] = min(lo[1], cy); lo[2] = min(lo[2], cz);
             hi[0] = max(hi[0], cx); hi[1] = max(hi[1], cy); hi[2] = max(hi[2], cz);
         }
@@ -2371,6 +2393,11 @@ __global__ void k_refresh(uint32_t* __restrict__ nodes, uint64_t n_words, uint32
 // levels 0..8 (256^3 words), which in turn beat levels 0..7 (1.54 -> 1.43).
 static uint32_t top_levels(uint32_t D) { return D < 3u ? 0u : std::min(10u, D); }
 
+static size_t top_words(uint32_t T0) {
+    const size_t side = top_side(T0);
+    return T0 ? side * side * side : 0;
+}
+
 static int build_top(ve_ctx* c, SceneSlot& s) {
     const uint32_t T0 = top_levels(s.depth);
     c->scenes_dirty = true;
@@ -2379,7 +2406,7 @@ static int build_top(ve_ctx* c, SceneSlot& s) {
         s.clip_hi[a] = 1e30f;
     }
     if (T0 == 0) return VE_OK;
-    const size_t n = size_t(1) << (3u * (T0 - 1u));
+    const size_t n = top_words(T0);
     if (!s.top) {
         if (cudaMalloc(&s.top, n * 4) != cudaSuccess) return fail(VE_ERR_NOMEM, "scene: top table allocation failed");
     }
@@ -3202,6 +3229,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
             if (pass <= max_b) {
                 if (em) {
                     if (count) k_trace<true, true><<<c->grid_trace_count, 256, 0, st>>>(a, pass);
+                    else if (flat) k_trace<false, true, true><<<c->grid_trace, 256, 0, st>>>(a, pass);
                     else k_trace<false, true><<<c->grid_trace, 256, 0, st>>>(a, pass);
                 } else {
                     if (count) k_trace<true><<<c->grid_trace_count, 256, 0, st>>>(a, pass);
@@ -3746,8 +3774,8 @@ static int build_scene_words(ve_ctx* c, const uint32_t* xyzm, uint64_t n, uint32
     };
     auto empty_scene = [&]() -> int {  // no voxel: OctreeCPU has no root, Octree::set keeps 8 zero words
         void* a = nullptr;
-        if (cudaMalloc(&a, 16 * 4) != cudaSuccess) return fail(VE_ERR_NOMEM, "scene_build: allocation failed");
-        VE_CUDA(cudaMemsetAsync(a, 0, 16 * 4, st));
+        if (cudaMalloc(&a, (8 + kNodePad) * 4) != cudaSuccess) return fail(VE_ERR_NOMEM, "scene_build: allocation failed");
+        VE_CUDA(cudaMemsetAsync(a, 0, (8 + kNodePad) * 4, st));
         VE_CUDA(cudaStreamSynchronize(st));
         *alloc = a;
         *words = reinterpret_cast<uint32_t*>(a) + 7;
@@ -3841,10 +3869,10 @@ static int build_scene_words(ve_ctx* c, const uint32_t* xyzm, uint64_t n, uint32
     // 4. words
     const uint64_t size = 9ull + 8ull * M;
     void* a = nullptr;
-    if (cudaMalloc(&a, (size + 8) * 4) != cudaSuccess)
+    if (cudaMalloc(&a, (size + kNodePad) * 4) != cudaSuccess)
         return fail(VE_ERR_NOMEM, "scene_build: node array allocation failed");
     uint32_t* w = reinterpret_cast<uint32_t*>(a) + 7;
-    cudaMemsetAsync(a, 0, (size + 8) * 4, st);
+    cudaMemsetAsync(a, 0, (size + kNodePad) * 4, st);
     k_root_word<<<1, 1, 0, st>>>(uint32_t(lv[2].m), w);
     for (uint32_t l = 2; l <= D + 1; l++) {
         const bool leaf = l == D + 1;
@@ -3937,7 +3965,7 @@ int ve_scene_upload(ve_ctx* c, const uint32_t* words, uint64_t n_words, uint32_t
     s.n_words = n_words;
     // nodes start 7 words into the allocation so every 8-child block
     // (slots 1 + 8k) begins on a 32-byte boundary
-    if (cudaMalloc(&s.alloc, (n_words + 8) * 4) != cudaSuccess)
+    if (cudaMalloc(&s.alloc, (n_words + kNodePad) * 4) != cudaSuccess)
         return fail(VE_ERR_NOMEM, "scene_upload: node array allocation failed");
     s.nodes = reinterpret_cast<uint32_t*>(s.alloc) + 7;
     const size_t cache_bytes = sizeof(CacheEntry) << c->cfg.hash_log2;
@@ -3946,6 +3974,7 @@ int ve_scene_upload(ve_ctx* c, const uint32_t* words, uint64_t n_words, uint32_t
         return fail(VE_ERR_NOMEM, "scene_upload: radiance cache allocation failed");
     }
     VE_CUDA(cudaMemcpyAsync(s.nodes, words, n_words * 4, cudaMemcpyHostToDevice, c->stream));
+    VE_CUDA(cudaMemsetAsync(s.nodes + n_words, 0, 8 * 4, c->stream));
     VE_CUDA(cudaMemsetAsync(s.cache, 0, cache_bytes, c->stream));
     s.live = true;
     if (int rc = build_top(c, s)) {
@@ -4114,8 +4143,8 @@ int ve_scene_footprint(ve_ctx* c, int32_t id, uint64_t* bytes) {
     if (!c || !bytes || id < 0 || size_t(id) >= c->scenes.size() || !c->scenes[id].live)
         return fail(VE_ERR_NOT_FOUND, "scene_footprint: unknown scene");
     const SceneSlot& sl = c->scenes[id];
-    const uint64_t top = sl.top_level ? (4ull << (3u * (sl.top_level - 1u))) : 0ull;
-    *bytes = (sl.n_words + 8) * 4 + (sizeof(CacheEntry) << c->cfg.hash_log2) + top;
+    const uint64_t top = 4ull * top_words(sl.top_level);
+    *bytes = (sl.n_words + kNodePad) * 4 + (sizeof(CacheEntry) << c->cfg.hash_log2) + top;
     return VE_OK;
 }
 
