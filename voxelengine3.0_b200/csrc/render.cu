@@ -58,7 +58,7 @@ struct DevScene {
     uint32_t cache_log2;
     uint32_t probes;
     uint32_t top_level;   // T0: levels 0..T0-1 resolved by the top table (0: none)
-    const uint32_t* top;  // top table, top_side(T0)^3 words
+    const uint32_t* top;  // top table, top_side(T0)^2 rows of top_row(T0) words
     // emissive lights (VE_FRAME_EMISSIVE; null until the scene's first such frame)
     EmLight* em_list;     // the registry, kEmCapacity records
     uint32_t* em_claim;   // claim table of registered (or dropped) light vids
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(256, 6) k_trace(FrameArgs a, uint32_t pass) {
     const uint32_t* nodes = nullptr;
     const uint32_t* top = nullptr;
     uint32_t n_words = 0;
-    float Lf = 0.0f;  // FLAT: 2^D, and the table's side in T0
+    FlatScene fs{};
     Dda s;
     FlatRay fr;
     Hit h;
@@ -492,17 +492,15 @@ __global__ void __launch_bounds__(256, 6) k_trace(FrameArgs a, uint32_t pass) {
                 const uint32_t p = e & 0x3FFFFFFFu;
                 const DevView& v = a.views[en.y];
                 const DevScene& S = a.scenes[v.scene];
-                nodes = S.nodes;
                 const f3 o = ld3(a.p_ray_o[p]);
                 f3 d = (e >> 31) ? mk(v.sun[0], v.sun[1], v.sun[2]) : ld3(a.p_ray_d[p]);
                 if (EM && (e >> 31) && (v.flags & VE_FRAME_EMISSIVE)) d = ld3(a.p_sdir[p]);
                 bool go;
                 if (FLAT) {
-                    T0 = top_side(S.top_level);
-                    top = flat_top(S.top, T0);
-                    Lf = float(1u << S.depth);
-                    go = flat_init(fr, o, d, v.cc_bounce, Lf);
+                    fs = flat_scene(S.nodes, S.top, S.depth);
+                    go = flat_init(fr, o, d, v.cc_bounce, fs.Lf);
                 } else {
+                    nodes = S.nodes;
                     n_words = word_bound(S.n_words);
                     D = S.depth;
                     top = S.top;
@@ -530,7 +528,7 @@ __global__ void __launch_bounds__(256, 6) k_trace(FrameArgs a, uint32_t pass) {
         const int lim = drained ? 0 : 32 - int(a.refill);
         while (__popc(__ballot_sync(0xffffffffu, state == kWalking)) > lim) {
             if (state == kWalking) {
-                if (FLAT) state = flat_step<true, true>(fr, nodes, top, T0, Lf);
+                if (FLAT) state = flat_step<true, true>(fr, fs);
                 else if (dda_step<COUNT, true, true>(s, nodes, n_words, D, top, T0, h, rc)) state = h.status;
             }
         }
@@ -2237,38 +2235,98 @@ static int sync_scenes(ve_ctx* c) {
 // found by walking levels 0..T0-1 of the node words exactly as the descent
 // does (out-of-range words read as zero).
 //
+// One thread per run of 8 cells along z, aligned, so that they share all but
+// the last three levels of their walk: those levels are walked once, the last
+// three as the tree they are (at most 7 words instead of 24), and the run is
+// one 32-byte store.  Bound by the writes of the table (556 MB at depth 10).
+// The last run of a row (the layer at 2^D) and tables under 8 cells walk cell
+// by cell.
+//
 // Also the box of the cells that can hold a voxel: a descent that ends above
 // level D steps over an empty cell (only level-D words are tested for a
 // material), so only cells internal down to level T0 can be hit.  box[0..2]
 // = smallest, box[3..5] = largest such cell coordinate (box[0] > box[3]: no
 // such cell).  Positions with a coordinate equal to 2^D (the last layer of
 // cells on each axis) are left out of the box; k_face_hits covers them.
-__global__ void k_build_top(const uint32_t* __restrict__ nodes, uint64_t n_words, uint32_t D, uint32_t T0,
-                            uint32_t* __restrict__ top, uint32_t* __restrict__ box) {
+__global__ void __launch_bounds__(256) k_build_top(const uint32_t* __restrict__ nodes, uint64_t n_words, uint32_t D,
+                                                   uint32_t T0, uint32_t* __restrict__ top, uint32_t* __restrict__ box) {
     __shared__ uint32_t sb[6];
     if (threadIdx.x < 6) sb[threadIdx.x] = threadIdx.x < 3 ? 0xFFFFFFFFu : 0u;
-    const uint32_t side = top_side(T0), n = side * side * side;
-    const uint32_t sh = D - T0 + 1u, L = 1u << D;
+    const uint32_t side = top_side(T0), row = top_row(T0), runs = row / 8u - 1u;  // the row's last 8 words are padding
+    const uint32_t sh = D - T0 + 1u, L = 1u << D, n = side * side * runs;
+    const uint32_t nw = uint32_t(n_words);
     uint32_t lo[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, hi[3] = {0u, 0u, 0u};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t cz = i % side, cy = (i / side) % side, cx = i / (side * side);
+        const uint32_t q = i / runs, cz = (i - q * runs) * 8u, cy = q / side, cx = q - cy * side;
         const uint32_t x = cx << sh, y = cy << sh, z = cz << sh;
-        uint32_t base = 0, ent = 0;
-        bool terminal = false;
-        for (uint32_t k = 0; k < T0; k++) {
-            const uint32_t raw = dev::fetch_node(nodes, n_words, base + locate(x, y, z, L >> k));
-            if (!(raw & 1u)) {
-                ent = ((L >> k) - 1u) << 1;
-                terminal = true;
-                break;
+        uint32_t e[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+        if (cz + 8u < side) {
+            uint32_t base = 0, k = 0;
+            bool in = true;
+            for (; k + 3u < T0 && in; k++) {
+                const uint32_t raw = dev::fetch_node(nodes, n_words, base + locate(x, y, z, L >> k));
+                in = (raw & 1u) != 0u;
+                if (in) base = raw >> 4;
             }
-            base = raw >> 4;
+            if (!in) {
+                const uint32_t ent = ((L >> (k - 1u)) - 1u) << 1;
+#pragma unroll
+                for (uint32_t c = 0; c < 8; c++) e[c] = ent;
+            } else {  // k = T0 - 3: the level of the run's 8-cell node
+#pragma unroll
+                for (uint32_t a = 0; a < 2; a++) {
+                    // the 8-cell node's two halves, each its own word at level T0-3
+                    const uint32_t za = (cz + 4u * a) << sh;
+                    const uint32_t ra = dev::fetch_node(nodes, n_words, base + locate(x, y, za, L >> k));
+#pragma unroll
+                    for (uint32_t b = 0; b < 2; b++) {
+                        const uint32_t zb = (cz + 4u * a + 2u * b) << sh;
+                        uint32_t rb = 0u;
+                        if (ra & 1u) rb = dev::fetch_node(nodes, n_words, (ra >> 4) + locate(x, y, zb, L >> (k + 1u)));
+#pragma unroll
+                        for (uint32_t c = 0; c < 2; c++) {
+                            const uint32_t zc = (cz + 4u * a + 2u * b + c) << sh;
+                            uint32_t ent;
+                            if (!(ra & 1u)) ent = ((L >> k) - 1u) << 1;
+                            else if (!(rb & 1u)) ent = ((L >> (k + 1u)) - 1u) << 1;
+                            else {
+                                const uint32_t rc = dev::fetch_node(nodes, n_words,
+                                                                    (rb >> 4) + locate(x, y, zc, L >> (k + 2u)));
+                                // a block past the end reads as the zero words that follow the array
+                                ent = (rc & 1u) ? ((min(rc >> 4, nw) << 1) | 1u) : ((L >> (k + 2u)) - 1u) << 1;
+                            }
+                            e[4u * a + 2u * b + c] = ent;
+                        }
+                    }
+                }
+            }
+        } else {
+#pragma unroll 1
+            for (uint32_t c = 0; c < 8u && cz + c < side; c++) {
+                uint32_t base = 0, ent = 0;
+                bool in = true;
+                for (uint32_t k = 0; k < T0 && in; k++) {
+                    const uint32_t raw = dev::fetch_node(nodes, n_words, base + locate(x, y, (cz + c) << sh, L >> k));
+                    in = (raw & 1u) != 0u;
+                    if (in) base = raw >> 4;
+                    else ent = ((L >> k) - 1u) << 1;
+                }
+                if (in) ent = (min(base, nw) << 1) | 1u;
+#pragma unroll
+                for (uint32_t j = 0; j < 8; j++)
+                    if (j == c) e[j] = ent;
+            }
         }
-        // a block past the end reads as the zero words that follow the array
-        top[i] = terminal ? ent : ((min(base, uint32_t(n_words)) << 1) | 1u);
-        if (!terminal && max(max(cx, cy), cz) + 1u < side) {
-            lo[0] = min(lo[0], cx); lo[1] = min(lo[1], cy); lo[2] = min(lo[2], cz);
-            hi[0] = max(hi[0], cx); hi[1] = max(hi[1], cy); hi[2] = max(hi[2], cz);
+        uint32_t* dst = top + size_t(q) * row + cz;
+        reinterpret_cast<uint4*>(dst)[0] = make_uint4(e[0], e[1], e[2], e[3]);
+        reinterpret_cast<uint4*>(dst)[1] = make_uint4(e[4], e[5], e[6], e[7]);
+        uint32_t inner = 0;
+#pragma unroll
+        for (uint32_t c = 0; c < 8; c++) inner |= (e[c] & 1u) << c;
+        if (cz + 8u >= side) inner &= (1u << (side - 1u - cz)) - 1u;  // without the layer at 2^D
+        if (inner && max(cx, cy) + 1u < side) {
+            lo[0] = min(lo[0], cx); lo[1] = min(lo[1], cy); lo[2] = min(lo[2], cz + uint32_t(__ffs(inner)) - 1u);
+            hi[0] = max(hi[0], cx); hi[1] = max(hi[1], cy); hi[2] = max(hi[2], cz + 31u - uint32_t(__clz(inner)));
         }
     }
     __syncthreads();
@@ -2288,22 +2346,20 @@ __global__ void k_build_top(const uint32_t* __restrict__ nodes, uint64_t n_words
 // the level-0 read to root words 1..7 instead of word 0 (internal.glsl's
 // locate at octreeLength).  Sets *hit when any integer position on the three
 // faces {x, y or z = 2^D} ends its descent on a material voxel — the only
-// positions outside the top table's cells that can be hit.
+// positions outside the box's cells that can be hit.  The descent starts from
+// the top table's layer at 2^D.
 __global__ void __launch_bounds__(256) k_face_hits(const uint32_t* __restrict__ nodes, uint64_t n_words, uint32_t D,
-                                                   uint32_t* hit) {
+                                                   uint32_t T0, const uint32_t* __restrict__ top, uint32_t* hit) {
     const uint32_t L = 1u << D, side = L + 1u;
-    const uint64_t per_face = uint64_t(side) * side;
     bool any = false;
-    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < 3u * per_face;
-         i += uint64_t(gridDim.x) * blockDim.x) {
-        const uint32_t f = uint32_t(i / per_face);
-        const uint64_t j = i % per_face;
-        const uint32_t u = uint32_t(j / side), v = uint32_t(j % side);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 3u * side * side; i += gridDim.x * blockDim.x) {
+        const uint32_t f = i / (side * side), j = i - f * (side * side);
+        const uint32_t u = j / side, v = j - u * side;
         const uint32_t x = f == 0 ? L : u, y = f == 1 ? L : (f == 0 ? u : v), z = f == 2 ? L : v;
-        // the descent of dda_step without the top table
-        uint32_t base = 0;
-        bool internal = true;
-        for (uint32_t k = 0; k < D && internal; k++) {
+        const uint32_t ent = __ldg(top + top_index(x, y, z, D, T0));
+        uint32_t base = ent >> 1;
+        bool internal = (ent & 1u) != 0u;
+        for (uint32_t k = T0; k < D && internal; k++) {
             const uint32_t b = D - k;
             const uint32_t raw = dev::fetch_node(nodes, n_words,
                                                  base + ((((x >> b) & 1u) << 2) | (((y >> b) & 1u) << 1) | ((z >> b) & 1u)));
@@ -2389,13 +2445,12 @@ __global__ void k_refresh(uint32_t* __restrict__ nodes, uint64_t n_words, uint32
 // Levels resolved by the top table: every level above the leaves up to
 // depth 10 (levels 0..D-1: a descent is one table word, then the leaf word),
 // levels 0..9 deeper down, none under depth 3.  At depth 10 the table is
-// 512^3 words (512 MiB): trace 1.084 -> 1.017 ms per 1080p frame against
+// 513 x 513 x 528 words (530 MiB): trace 1.084 -> 1.017 ms per 1080p frame against
 // levels 0..8 (256^3 words), which in turn beat levels 0..7 (1.54 -> 1.43).
 static uint32_t top_levels(uint32_t D) { return D < 3u ? 0u : std::min(10u, D); }
 
 static size_t top_words(uint32_t T0) {
-    const size_t side = top_side(T0);
-    return T0 ? side * side * side : 0;
+    return T0 ? size_t(top_side(T0)) * top_side(T0) * top_row(T0) : 0;
 }
 
 static int build_top(ve_ctx* c, SceneSlot& s) {
@@ -2418,7 +2473,7 @@ static int build_top(ve_ctx* c, SceneSlot& s) {
     cudaMemcpyAsync(d_box, init, sizeof(init), cudaMemcpyHostToDevice, c->stream);
     k_build_top<<<c->num_sms * 8, 256, 0, c->stream>>>(s.nodes, s.n_words, s.depth, T0, s.top, d_box);
     // faces of more than 3 * 4097^2 positions are not searched: no box then
-    if (s.depth <= 12) k_face_hits<<<c->num_sms * 8, 256, 0, c->stream>>>(s.nodes, s.n_words, s.depth, d_box + 6);
+    if (s.depth <= 12) k_face_hits<<<c->num_sms * 8, 256, 0, c->stream>>>(s.nodes, s.n_words, s.depth, T0, s.top, d_box + 6);
     cudaMemcpyAsync(box, d_box, sizeof(box), cudaMemcpyDeviceToHost, c->stream);
     const cudaError_t e = cudaStreamSynchronize(c->stream);
     cudaFree(d_box);
