@@ -218,6 +218,7 @@ struct FrameArgs {
     uint2* shade_list;      // {vid, pixel} per path
     uint32_t shade_cap;
     float* rank;            // the scene's {t_high, t_mid, histogram[256]} (thresholds from the previous frame)
+    FlatScene one;          // the batch's scene when all its views share one whose table reaches the leaves
 };
 
 constexpr uint32_t kRankBins = 256;
@@ -425,10 +426,18 @@ __global__ void __launch_bounds__(256) k_decay(CacheEntry* cache, uint32_t n, fl
 // EM: the batch has VE_FRAME_EMISSIVE views (shadow rays toward lights).
 // FLAT: every scene of the batch has a top table reaching its leaves (T0 = D):
 // flat_step.  Fetch-counting batches take the general walk.
+// ONE: the batch has one such scene, whose pointers and size then come from
+// the kernel's arguments instead of seven registers of every lane: 32
+// registers and 8 CTAs/SM (0.637 -> 0.606 ms of trace per 1080p depth-10 frame;
+// at 6 CTAs/SM 0.641, so it is the resident warps that pay: the walk waits on
+// its loads).
+// A warp's first 32 rays are fixed: with 9472 warps at the cursor from the
+// start, the trace of a 256x256 depth-7 frame took 0.056 ms instead of 0.047.
 enum : uint32_t { kLaneIdle = 4u };  // lane state: kWalking, a finished ray's status to be stored, or no ray
-template <bool COUNT, bool EM = false, bool FLAT = false>
-__global__ void __launch_bounds__(256, 6) k_trace(FrameArgs a, uint32_t pass) {
-    static_assert(!(COUNT && FLAT), "fetch counts need the walk of every level");
+template <bool COUNT, bool EM = false, bool FLAT = false, bool ONE = false>
+__global__ void __launch_bounds__(256, ONE ? 8 : 6) k_trace(FrameArgs a, uint32_t pass) {
+    static_assert(!(COUNT && FLAT) && (FLAT || !ONE), "fetch counts need the walk of every level");
+    __shared__ uint32_t entry[256];  // the queue entry of each lane's ray, until its result is stored
     // the pass's extension rays, then its shadow rays: warps stay mostly of
     // one kind, and the shorter shadow rays form the tail of the pass
     const uint32_t n_ext = a.counters[CNT_RAY + pass];
@@ -436,19 +445,25 @@ __global__ void __launch_bounds__(256, 6) k_trace(FrameArgs a, uint32_t pass) {
     uint32_t* cursor = &a.counters[CNT_CURSOR + pass];
     const uint32_t lane = lane_id();
     bool drained = false;  // warp-uniform: every ray of the pass has been handed out
+    // the first 32 rays of each warp are its own, so a pass with less than a
+    // grid of them touches no cursor; the cursor hands out the rest
+    const uint32_t own = gridDim.x * blockDim.x;
+    uint32_t first_idx = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;
+    bool first = true;
     uint32_t state = kLaneIdle;
-    uint32_t e = 0, D = 0, T0 = 0;
+    uint32_t D = 0, T0 = 0;
     const uint32_t* nodes = nullptr;
     const uint32_t* top = nullptr;
     uint32_t n_words = 0;
     FlatScene fs{};
+    if (ONE) fs = a.one;
     Dda s;
     FlatRay fr;
     Hit h;
     RayCount rc;
     for (;;) {
         if (state < kWalking) {  // store a finished ray's result
-            const uint32_t p = e & 0x3FFFFFFFu;
+            const uint32_t e = entry[threadIdx.x], p = e & 0x3FFFFFFFu;
             const uint32_t word = FLAT ? fr.blk : h.id;
             const uint32_t x = FLAT ? fr.bx - kPosBits : h.x, y = FLAT ? fr.by - kPosBits : h.y,
                            z = FLAT ? fr.bz - kPosBits : h.z;
@@ -479,17 +494,19 @@ __global__ void __launch_bounds__(256, 6) k_trace(FrameArgs a, uint32_t pass) {
         if (drained) break;  // the last rays have just been stored
         const unsigned idle = __ballot_sync(0xffffffffu, state == kLaneIdle);
         const uint32_t want = uint32_t(__popc(idle));
-        const int leader = __ffs(idle) - 1;
-        uint32_t first_idx = 0;
-        if (int(lane) == leader) first_idx = atomicAdd(cursor, want);
-        first_idx = __shfl_sync(0xffffffffu, first_idx, leader);
-        drained = first_idx + want >= n;
+        if (!first) {
+            const int leader = __ffs(idle) - 1;
+            if (int(lane) == leader) first_idx = own + atomicAdd(cursor, want);
+            first_idx = __shfl_sync(0xffffffffu, first_idx, leader);
+        }
+        drained = first ? own >= n : first_idx + want >= n;
+        first = false;
         if (state == kLaneIdle) {
             const uint32_t idx = first_idx + uint32_t(__popc(idle & ((1u << lane) - 1u)));
             if (idx < n) {
                 const uint2 en = idx < n_ext ? a.rayq[idx] : a.rayq_sh[idx - n_ext];
-                e = en.x;
-                const uint32_t p = e & 0x3FFFFFFFu;
+                const uint32_t e = en.x, p = e & 0x3FFFFFFFu;
+                entry[threadIdx.x] = e;
                 const DevView& v = a.views[en.y];
                 const DevScene& S = a.scenes[v.scene];
                 const f3 o = ld3(a.p_ray_o[p]);
@@ -497,7 +514,7 @@ __global__ void __launch_bounds__(256, 6) k_trace(FrameArgs a, uint32_t pass) {
                 if (EM && (e >> 31) && (v.flags & VE_FRAME_EMISSIVE)) d = ld3(a.p_sdir[p]);
                 bool go;
                 if (FLAT) {
-                    fs = flat_scene(S.nodes, S.top, S.depth);
+                    if (!ONE) fs = flat_scene(S.nodes, S.top, S.depth);
                     go = flat_init(fr, o, d, v.cc_bounce, fs.Lf);
                 } else {
                     nodes = S.nodes;
@@ -2158,8 +2175,8 @@ struct ve_ctx {
     ve_frame_config split_frame{};  // the last split frame's config
     ve::DevBuf<float> ray_in;      // ve_raycast_batch: origins and directions
     ve::DevBuf<uint32_t> ray_out;  // ve_raycast_batch: 8 words per ray
-    int grid_trace = 0, grid_trace_count = 0, grid_shade = 0;
-    int occ_trace = 1, occ_trace_count = 1, occ_shade = 1;  // occupancy maxima (blocks/SM)
+    int grid_trace = 0, grid_trace_one = 0, grid_trace_count = 0, grid_shade = 0;
+    int occ_trace = 1, occ_trace_one = 1, occ_trace_count = 1, occ_shade = 1;  // occupancy maxima (blocks/SM)
     int occ_shade_mode[8] = {1, 1, 1, 1, 1, 1, 1, 1};       // ... per shading instance (kModeEm | kModeLb | kModeNrc)
     int occ_emit_mode[4] = {1, 1, 1, 1};                    // ... per scheduled-emit instance
     ve_launch_config launch{0, 0, ve::kDefaultRefill, 0};
@@ -2805,6 +2822,7 @@ static void collect_all_timing(ve_ctx* c) {
 static void apply_launch(ve_ctx* c) {
     auto pick = [&](uint32_t want, int occ) { return int((want == 0 || int(want) > occ) ? occ : int(want)); };
     c->grid_trace = c->num_sms * pick(c->launch.trace_blocks_per_sm, c->occ_trace);
+    c->grid_trace_one = c->num_sms * pick(c->launch.trace_blocks_per_sm, c->occ_trace_one);
     c->grid_trace_count = c->num_sms * pick(c->launch.trace_blocks_per_sm, c->occ_trace_count);
     c->grid_shade = c->num_sms * pick(c->launch.shade_blocks_per_sm, c->occ_shade);
     // default: refill when 20 of 32 lanes are idle (measured on the depth-10
@@ -2878,6 +2896,22 @@ static void fill_view(DevView& d, const ve_view& v) {
     d.lb = LbParams{f.time, f.update_time, f.disable_stale_reset, f.sample_cap_direct, f.sample_cap_indirect,
                     f.firefly_k, f.firefly_floor};
     set_rows(d, f, (f.flags & VE_FRAME_SPLIT) != 0);
+}
+
+static void launch_trace(const ve_ctx* c, cudaStream_t st, const FrameArgs& a, uint32_t pass, bool count, bool em,
+                         bool flat, bool one) {
+    const uint32_t g = uint32_t(count ? c->grid_trace_count : one ? c->grid_trace_one : c->grid_trace);
+    if (em) {
+        if (count) k_trace<true, true><<<g, 256, 0, st>>>(a, pass);
+        else if (one) k_trace<false, true, true, true><<<g, 256, 0, st>>>(a, pass);
+        else if (flat) k_trace<false, true, true><<<g, 256, 0, st>>>(a, pass);
+        else k_trace<false, true><<<g, 256, 0, st>>>(a, pass);
+    } else {
+        if (count) k_trace<true><<<g, 256, 0, st>>>(a, pass);
+        else if (one) k_trace<false, false, true, true><<<g, 256, 0, st>>>(a, pass);
+        else if (flat) k_trace<false, false, true><<<g, 256, 0, st>>>(a, pass);
+        else k_trace<false><<<g, 256, 0, st>>>(a, pass);
+    }
 }
 
 static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_outputs* outs) {
@@ -3047,8 +3081,10 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
     // per-path NEE records and the registry commit's sort buffers
     // the trace's FLAT instance: every view's scene has a top table reaching
     // its leaves (depth 3..10)
-    bool flat = true;
+    // ... and its one-scene form: all of them show the same scene
+    bool flat = true, one = true;
     for (uint32_t i = 0; i < nv; i++) {
+        one = one && views[i].scene_id == views[0].scene_id;
         const SceneSlot& sc = c->scenes[views[i].scene_id];
         flat = flat && sc.top_level != 0u && sc.top_level == sc.depth;
     }
@@ -3224,6 +3260,11 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         a.p_res = c->p_res.p;
         a.res_list = c->res_list.p;
     }
+    one = one && flat;
+    if (one) {
+        const SceneSlot& sc = c->scenes[views[0].scene_id];
+        a.one = flat_scene(sc.nodes, sc.top, sc.depth);
+    }
     const bool em = (flags & VE_FRAME_EMISSIVE) != 0;
     const bool lbm = (flags & VE_FRAME_LBUFFER) != 0;
     const bool nrcm = (flags & (VE_FRAME_LEARNED | VE_FRAME_TERMINATE_HASH | VE_FRAME_TRAIN)) != 0;
@@ -3282,15 +3323,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
             }
             rec();
             if (pass <= max_b) {
-                if (em) {
-                    if (count) k_trace<true, true><<<c->grid_trace_count, 256, 0, st>>>(a, pass);
-                    else if (flat) k_trace<false, true, true><<<c->grid_trace, 256, 0, st>>>(a, pass);
-                    else k_trace<false, true><<<c->grid_trace, 256, 0, st>>>(a, pass);
-                } else {
-                    if (count) k_trace<true><<<c->grid_trace_count, 256, 0, st>>>(a, pass);
-                    else if (flat) k_trace<false, false, true><<<c->grid_trace, 256, 0, st>>>(a, pass);
-                    else k_trace<false><<<c->grid_trace, 256, 0, st>>>(a, pass);
-                }
+                launch_trace(c, st, a, pass, count, em, flat, one);
                 launches++;
                 trace_launches++;
             }
@@ -3370,7 +3403,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
                                      flags & (VE_FRAME_COUNT_FETCH | VE_FRAME_PATH_RGB | VE_FRAME_LEARNED |
                                               VE_FRAME_TERMINATE_HASH | VE_FRAME_TRAIN | VE_FRAME_SCHEDULED |
                                               VE_FRAME_EMISSIVE | VE_FRAME_LBUFFER | VE_FRAME_SPLIT),
-                                     paths, uint64_t(c->grid_trace), uint64_t(c->grid_shade),
+                                     paths, uint64_t(c->grid_trace), uint64_t(c->grid_trace_one), uint64_t(c->grid_shade),
                                      uint64_t(c->launch.refill_threshold), uint64_t(uintptr_t(nrc)),
                                      uint64_t(a.nrc_ready)};
         for (auto& d : decays) {
@@ -3381,6 +3414,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         for (int sc : em_scenes) key.push_back((1ull << 62) | uint64_t(uint32_t(sc)));
         key.push_back((1ull << 61) | uint64_t(parity));
         key.push_back((1ull << 59) | uint64_t(flat));
+        if (one) key.push_back((1ull << 58) | uint64_t(uint32_t(views[0].scene_id)));  // its pointers are captured
         key.push_back((1ull << 60) | (uint64_t(set) << 8) | uint64_t(part));
         ve_ctx::GraphEntry* ge = nullptr;
         for (auto& g : c->graphs)
@@ -3656,10 +3690,12 @@ int ve_ctx_create(const ve_renderer_config* cfg, ve_ctx** out) {
             return fail(VE_ERR_CUDA, "ctx_create: constant table upload failed");
         }
     }
-    int bt = 0, btc = 0, bs = 0;
+    int bt = 0, bt1 = 0, btc = 0, bs = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt, k_trace<false>, 256, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&btc, k_trace<true>, 256, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bs, k_shade<0>, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt1, k_trace<false, false, true, true>, 256, 0);
+    x->occ_trace_one = std::max(bt1, 1);
     x->occ_trace = std::max(bt, 1);
     x->occ_trace_count = std::max(btc, 1);
     x->occ_shade = std::max(bs, 1);
@@ -4505,12 +4541,12 @@ int ve_autotune(ve_ctx* c, const ve_view* views, uint32_t nv, uint32_t frames, v
         *ms = (c->tot_ms[0] - t0) / float(frames);
         return VE_OK;
     };
-    ve_launch_config cur{uint32_t(c->occ_trace), uint32_t(c->occ_shade), ve::kDefaultRefill, 0};
+    ve_launch_config cur{uint32_t(c->occ_trace_one), uint32_t(c->occ_shade), ve::kDefaultRefill, 0};
     float best_ms = 0.0f;
     int rc = measure(cur, &best_ms);
     if (rc) return rc;
     // coordinate descent: trace blocks/SM, shade blocks/SM, refill threshold
-    for (int tb = 1; tb <= c->occ_trace; tb++) {
+    for (int tb = 1; tb <= c->occ_trace_one; tb++) {
         ve_launch_config t = cur;
         t.trace_blocks_per_sm = uint32_t(tb);
         float ms = 0;
