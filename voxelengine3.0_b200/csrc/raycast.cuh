@@ -221,8 +221,8 @@ __device__ __forceinline__ bool dda_step(Dda& s, const uint32_t* __restrict__ no
 //     a rising axis (low 22 bits all ones) and of -1.5 * 2^23 for a falling one
 //     (all zeros), ((b ^ c) & ~m) ^ c is the cell's last coordinate or its
 //     first one (m = cell size - 1), and adding c as a float gives the plane.
-//   * The cell is one mask m, compared with the changed bits of the position:
-//     no level, no leading-zero count.
+//   * The cell is its table entry, whose mask is compared with the changed bits
+//     of the position: no level, no leading-zero count.
 //   * min/max of three operands are one instruction each.  They return what
 //     the glm selects of dda_step return: inside the volume no exit distance
 //     is NaN (an axis with 1/d = +-inf has a non-zero numerator of its sign),
@@ -241,9 +241,8 @@ struct FlatRay {
     f3 o, d, inv;
     float t, t_end;
     uint32_t left;        // steps before the timeout
-    uint32_t bx, by, bz;  // biased position bits of the last step
-    uint32_t m;           // size - 1 of its cell
-    uint32_t blk;         // m = 0: its leaf block; after a hit: the leaf's word (WORD) or slot
+    uint32_t bx, by, bz;  // biased position bits
+    uint32_t ent;         // table entry of its cell; after a hit: the leaf's word (WORD) or slot
 };
 
 // Table pointer such that the index of the biased bits, modulo 2^32, lands on
@@ -287,16 +286,28 @@ __device__ __forceinline__ float flat_exit(uint32_t b, uint32_t m, float o, floa
     return ((plane - o) + e) * inv;
 }
 
-// Returns false when the ray misses the volume (escaped; `left` is then one
-// less than the checks allow).
+// The position at distance t: false when it lies outside (or, CLIP, t beyond
+// t_end).
+template <bool CLIP>
+__device__ __forceinline__ bool flat_at(const FlatRay& s, const FlatScene& w, uint32_t& bx, uint32_t& by, uint32_t& bz) {
+    const f3 r = add(muls(s.d, s.t), s.o);
+    const float lo = min3_nan(r.x, r.y, r.z), hi = max3_nan(r.x, r.y, r.z);
+    bx = __float_as_uint(__fadd_rz(r.x, kPosBias));
+    by = __float_as_uint(__fadd_rz(r.y, kPosBias));
+    bz = __float_as_uint(__fadd_rz(r.z, kPosBias));
+    return 0.0f <= lo && hi <= w.Lf && !(CLIP && s.t > s.t_end);
+}
+__device__ __forceinline__ uint32_t flat_entry(const FlatScene& w, uint32_t bx, uint32_t by, uint32_t bz) {
+    return __ldg(w.topb + (((by >> 1) * w.side + (bx >> 1)) * w.row + (bz >> 1)));
+}
+
+// The ray's set-up up to its first position's distance: false when it misses
+// the volume (escaped; `left` is then one less than the checks allow).
 __device__ __forceinline__ bool flat_init(FlatRay& s, f3 o, f3 d, uint32_t controlchecks, float Lf) {
     s.inv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
     s.d = d;
     s.o = add(o, muls(d, 4.0f));
     s.left = controlchecks + 1u;
-    s.bx = s.by = s.bz = 0u;  // no position yet: every bit differs from the first step's
-    s.m = 0u;
-    s.blk = 0u;
     s.t = 0.0f;
     if (!in_bounds(s.o, Lf)) {
         const f3 t1 = mul(mk((0.0f - s.o.x) + 0.001f, (0.0f - s.o.y) + 0.001f, (0.0f - s.o.z) + 0.001f), s.inv);
@@ -309,39 +320,50 @@ __device__ __forceinline__ bool flat_init(FlatRay& s, f3 o, f3 d, uint32_t contr
     }
     return true;
 }
-
-// One iteration of the reference loop: kWalking, or how the ray ended (kHit /
-// kEscaped / kTimeout).  WORD: a hit leaves the leaf's word in blk, else its
-// slot.  CLIP as in dda_step.
-template <bool WORD, bool CLIP>
-__device__ __forceinline__ uint32_t flat_step(FlatRay& s, const FlatScene& w) {
-    const f3 r = add(muls(s.d, s.t), s.o);
-    const float lo = min3_nan(r.x, r.y, r.z), hi = max3_nan(r.x, r.y, r.z);
-    if (!(0.0f <= lo && hi <= w.Lf) || (CLIP && s.t > s.t_end)) return kEscaped;
+// The first position's checks and table entry: kWalking, or how the ray ended.
+template <bool CLIP>
+__device__ __forceinline__ uint32_t flat_first(FlatRay& s, const FlatScene& w) {
+    if (!flat_at<CLIP>(s, w, s.bx, s.by, s.bz)) return kEscaped;
     if (s.left == 0u) return kTimeout;
     s.left--;
-    const uint32_t bx = __float_as_uint(__fadd_rz(r.x, kPosBias));
-    const uint32_t by = __float_as_uint(__fadd_rz(r.y, kPosBias));
-    const uint32_t bz = __float_as_uint(__fadd_rz(r.z, kPosBias));
+    s.ent = flat_entry(w, s.bx, s.by, s.bz);
+    return kWalking;
+}
+
+// One iteration of the reference loop, from the lookup of the current
+// position's cell to the checks of the next one: kWalking, or how the ray
+// ended (kHit / kEscaped / kTimeout).  The cell's exit depends on its table
+// entry but not on its leaf word, so the next position's table entry is loaded
+// while the leaf word is on its way: a step waits for one load, not two (1080p
+// depth-10 frame: trace 0.594 -> 0.545 ms, primary 0.351 -> 0.324; 256x256
+// depth 7: 0.047 -> 0.042 and 0.0345 -> 0.0273).  A ray that hits has loaded
+// one entry in vain.
+// WORD: a hit leaves the leaf's word in ent, else its slot.  CLIP as in
+// dda_step.
+template <bool WORD, bool CLIP>
+__device__ __forceinline__ uint32_t flat_step(FlatRay& s, const FlatScene& w) {
+    const uint32_t blk = s.ent >> 1;
+    const bool leaf = (s.ent & 1u) != 0u;
+    const uint32_t m = leaf ? 0u : blk;  // size - 1 of the cell
+    const uint32_t off = blk + (((s.bx << 2) & 4u) | ((s.by << 1) & 2u) | (s.bz & 1u));
+    uint32_t raw = 0u;
+    if (leaf) raw = __ldg(w.nodes + off);
+    s.t = fminf(fminf(flat_exit(s.bx, m, s.o.x, s.inv.x), flat_exit(s.by, m, s.o.y, s.inv.y)),
+                flat_exit(s.bz, m, s.o.z, s.inv.z));
+    uint32_t bx, by, bz;
+    const bool in = flat_at<CLIP>(s, w, bx, by, bz);
     const uint32_t xd = (bx ^ s.bx) | (by ^ s.by) | (bz ^ s.bz);
-    s.bx = bx; s.by = by; s.bz = bz;
-    if (xd > s.m) {            // another cell
-        if (xd > (s.m | 1u)) {  // ... and not of the same leaf block
-            const uint32_t ent = __ldg(w.topb + (((by >> 1) * w.side + (bx >> 1)) * w.row + (bz >> 1)));
-            s.m = (ent & 1u) ? 0u : ent >> 1;
-            s.blk = ent >> 1;
-        }
-        if (s.m == 0u) {
-            const uint32_t off = s.blk + (((bx << 2) & 4u) | ((by << 1) & 2u) | (bz & 1u));
-            const uint32_t raw = __ldg(w.nodes + off);
-            if (raw & 254u) {
-                s.blk = WORD ? raw : off;
-                return kHit;
-            }
-        }
+    uint32_t ent = s.ent;
+    if (in && xd > (m | 1u)) ent = flat_entry(w, bx, by, bz);  // neither this cell nor its leaf block
+    if (raw & 254u) {
+        s.ent = WORD ? raw : off;
+        return kHit;
     }
-    s.t = fminf(fminf(flat_exit(bx, s.m, s.o.x, s.inv.x), flat_exit(by, s.m, s.o.y, s.inv.y)),
-                flat_exit(bz, s.m, s.o.z, s.inv.z));
+    if (!in) return kEscaped;
+    if (s.left == 0u) return kTimeout;
+    s.left--;
+    s.bx = bx; s.by = by; s.bz = bz;
+    s.ent = ent;
     return kWalking;
 }
 
@@ -356,14 +378,14 @@ __device__ __forceinline__ Hit raycast(const uint32_t* __restrict__ nodes, uint6
         h.status = kEscaped;
         h.id = h.material = h.x = h.y = h.z = h.size = 0;
         if (flat_init(s, o, d, controlchecks, w.Lf)) {
-            do h.status = flat_step<false, false>(s, w);
-            while (h.status == kWalking);
+            h.status = flat_first<false>(s, w);
+            while (h.status == kWalking) h.status = flat_step<false, false>(s, w);
         }
         // the reference's count includes the check that found no steps left
         h.checks = controlchecks + 1u - s.left + (h.status == kTimeout ? 1u : 0u);
         if (h.status == kHit) {
-            h.id = s.blk;
-            h.material = (__ldg(nodes + s.blk) & 254u) >> 1;
+            h.id = s.ent;
+            h.material = (__ldg(nodes + s.ent) & 254u) >> 1;
             h.x = s.bx - kPosBits; h.y = s.by - kPosBits; h.z = s.bz - kPosBits;
             h.size = 1u;
         }

@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(256, ONE ? 8 : 6) k_trace(FrameArgs a, uint32_
     for (;;) {
         if (state < kWalking) {  // store a finished ray's result
             const uint32_t e = entry[threadIdx.x], p = e & 0x3FFFFFFFu;
-            const uint32_t word = FLAT ? fr.blk : h.id;
+            const uint32_t word = FLAT ? fr.ent : h.id;
             const uint32_t x = FLAT ? fr.bx - kPosBits : h.x, y = FLAT ? fr.by - kPosBits : h.y,
                            z = FLAT ? fr.bz - kPosBits : h.z;
             if (e >> 31) {
@@ -524,7 +524,6 @@ __global__ void __launch_bounds__(256, ONE ? 8 : 6) k_trace(FrameArgs a, uint32_
                     T0 = S.top_level;
                     go = !dda_init(s, o, d, v.cc_bounce, D, h);
                 }
-                state = go ? kWalking : kEscaped;
                 // a bounce ray that escapes or times out shades as sky alike,
                 // so it ends on leaving the box of the cells that can hold a
                 // voxel (exit of its slab); shadow rays walk on (there a
@@ -539,6 +538,7 @@ __global__ void __launch_bounds__(256, ONE ? 8 : 6) k_trace(FrameArgs a, uint32_
                     te = gmin(gmin(tx, ty), tz);
                 }
                 fr.t_end = s.t_end = te;
+                state = !go ? kEscaped : FLAT ? flat_first<true>(fr, fs) : kWalking;
             }
         }
         // step until `refill` lanes are idle; run all out once drained
