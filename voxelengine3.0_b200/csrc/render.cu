@@ -545,7 +545,12 @@ __global__ void __launch_bounds__(256, ONE ? 8 : 6) k_trace(FrameArgs a, uint32_
         const int lim = drained ? 0 : 32 - int(a.refill);
         while (__popc(__ballot_sync(0xffffffffu, state == kWalking)) > lim) {
             if (state == kWalking) {
-                if (FLAT) state = flat_step<true, true>(fr, fs);
+                if (FLAT) {  // three steps per look at the warp's other lanes (trace 0.545 -> 0.520 ms per 1080p
+                             // depth-10 frame, two 0.530, four 0.520)
+                    state = flat_step<true, true>(fr, fs);
+                    if (state == kWalking) state = flat_step<true, true>(fr, fs);
+                    if (state == kWalking) state = flat_step<true, true>(fr, fs);
+                }
                 else if (dda_step<COUNT, true, true>(s, nodes, n_words, D, top, T0, h, rc)) state = h.status;
             }
         }
