@@ -3960,6 +3960,25 @@ int ve_ctx_join(ve_ctx* c) {
     return VE_OK;
 }
 
+int ve_host_alloc(uint64_t bytes, void** out) {
+    if (!out || bytes == 0) return fail(VE_ERR_INVALID, "host_alloc: null output or no bytes");
+    *out = nullptr;
+    if (cudaHostAlloc(out, bytes, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        *out = nullptr;
+        return fail(VE_ERR_NOMEM, "host_alloc: pinned allocation failed");
+    }
+    return VE_OK;
+}
+
+int ve_host_free(void* p) {
+    if (p && cudaFreeHost(p) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(VE_ERR_INVALID, "host_free: not a host_alloc block");
+    }
+    return VE_OK;
+}
+
 int ve_ctx_synchronize(ve_ctx* c) {
     if (!c) return fail(VE_ERR_INVALID, "ctx_synchronize: null context");
     VE_CUDA(cudaStreamSynchronize(c->stream));
