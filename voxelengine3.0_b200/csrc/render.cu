@@ -2180,6 +2180,7 @@ struct SceneSlot {
     // bounce-ray clip box (DevScene::clip_lo/hi), from the top table build;
     // unbounded when the scene has no top table
     float clip_lo[3] = {-1e30f, -1e30f, -1e30f}, clip_hi[3] = {1e30f, 1e30f, 1e30f};
+    uint32_t box[6] = {0, 0, 0, 0, 0, 0};  // the cells that can hold a voxel, as k_build_top found them
 };
 
 template <typename T>
@@ -2219,6 +2220,9 @@ struct FrameSet {
     ve::DevBuf<unsigned long long> stats;
     unsigned long long* h_stats = nullptr;  // pinned
 };
+
+// edits per call whose device lists stay allocated for the next call (12 MB)
+constexpr uint64_t kKeptEdits = 1u << 20;
 
 struct ve_ctx {
     int device = 0;
@@ -2303,6 +2307,8 @@ struct ve_ctx {
     int split_scene = -1;
     bool split_delta_clean = false;  // the per-frame table is all zeros (cleared by the last export)
     ve_frame_config split_frame{};  // the last split frame's config
+    ve::DevBuf<uint32_t> edit;     // ve_scene_apply_edits / _refresh: the caller's lists (kept up to kKeptEdits)
+    ve::DevBuf<uint32_t> box;      // build_top: the box, the face search's result
     ve::DevBuf<float> ray_in;      // ve_raycast_batch: origins and directions
     ve::DevBuf<uint32_t> ray_out;  // ve_raycast_batch: 8 words per ray
     int grid_trace = 0, grid_trace_one = 0, grid_trace_count = 0, grid_shade = 0;
@@ -2522,10 +2528,18 @@ __global__ void __launch_bounds__(256) k_face_hits(const uint32_t* __restrict__ 
 }
 
 // Octree::applyEdits upload (octree.cpp:228-314): words[i] -> nodes[slots[i]].
+// Sets *moved when a word changes what the top table holds of it: whether it
+// is internal, or an internal word's child block.  Digging, filling and
+// repainting voxels inside existing blocks changes leaf words and child counts
+// only, and then the table need not be rebuilt (223 us at depth 10).
 __global__ void k_scatter_words(uint32_t* __restrict__ nodes, const uint32_t* __restrict__ slots,
-                                const uint32_t* __restrict__ words, uint64_t n) {
-    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x)
-        nodes[slots[i]] = words[i];
+                                const uint32_t* __restrict__ words, uint64_t n, uint32_t* moved) {
+    bool m = false;
+    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
+        const uint32_t w = words[i], old = atomicExch(nodes + slots[i], w);  // (a slot may be listed twice)
+        m |= ((w ^ old) & 1u) != 0u || ((w & 1u) && (w >> 4) != (old >> 4));
+    }
+    if (__any_sync(0xFFFFFFFFu, m) && (threadIdx.x & 31u) == 0u) atomicOr(moved, 1u);
 }
 
 // Slot of the voxel leaf at (x, y, z) when it holds a material, else ~0u:
@@ -2600,31 +2614,40 @@ static size_t top_words(uint32_t T0) {
     return T0 ? size_t(top_side(T0)) * top_side(T0) * top_row(T0) : 0;
 }
 
-static int build_top(ve_ctx* c, SceneSlot& s) {
+// The scene's top table, clip box and face search; with `rebuild` false the
+// table and its box stand (the words they come from have not changed).
+static int build_top(ve_ctx* c, SceneSlot& s, bool rebuild = true) {
     const uint32_t T0 = top_levels(s.depth);
-    c->scenes_dirty = true;
+    const float was[6] = {s.clip_lo[0], s.clip_lo[1], s.clip_lo[2], s.clip_hi[0], s.clip_hi[1], s.clip_hi[2]};
     for (int a = 0; a < 3; a++) {  // unbounded until the table says otherwise
         s.clip_lo[a] = -1e30f;
         s.clip_hi[a] = 1e30f;
     }
+    if (rebuild) c->scenes_dirty = true;
     if (T0 == 0) return VE_OK;
     const size_t n = top_words(T0);
     if (!s.top) {
         if (cudaMalloc(&s.top, n * 4) != cudaSuccess) return fail(VE_ERR_NOMEM, "scene: top table allocation failed");
     }
     s.top_level = T0;
-    uint32_t* d_box = nullptr;
-    if (cudaMalloc(&d_box, 7 * 4) != cudaSuccess) return fail(VE_ERR_NOMEM, "scene: allocation failed");
+    if (int rc = c->box.ensure(8)) return rc;
+    uint32_t* d_box = c->box.p;
     const uint32_t init[7] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u};
     uint32_t box[7];
-    cudaMemcpyAsync(d_box, init, sizeof(init), cudaMemcpyHostToDevice, c->stream);
-    k_build_top<<<c->num_sms * 8, 256, 0, c->stream>>>(s.nodes, s.n_words, s.depth, T0, s.top, d_box);
+    if (rebuild) {
+        cudaMemcpyAsync(d_box, init, sizeof(init), cudaMemcpyHostToDevice, c->stream);
+        k_build_top<<<c->num_sms * 8, 256, 0, c->stream>>>(s.nodes, s.n_words, s.depth, T0, s.top, d_box);
+    } else {
+        cudaMemsetAsync(d_box + 6, 0, 4, c->stream);
+    }
     // faces of more than 3 * 4097^2 positions are not searched: no box then
-    if (s.depth <= 12) k_face_hits<<<c->num_sms * 8, 256, 0, c->stream>>>(s.nodes, s.n_words, s.depth, T0, s.top, d_box + 6);
+    if (s.depth <= 12)
+        k_face_hits<<<c->num_sms * 8, 256, 0, c->stream>>>(s.nodes, s.n_words, s.depth, T0, s.top, d_box + 6);
     cudaMemcpyAsync(box, d_box, sizeof(box), cudaMemcpyDeviceToHost, c->stream);
     const cudaError_t e = cudaStreamSynchronize(c->stream);
-    cudaFree(d_box);
     if (e != cudaSuccess) return fail(VE_ERR_CUDA, std::string("scene: top table build: ") + cudaGetErrorString(e));
+    if (rebuild) std::memcpy(s.box, box, sizeof(s.box));
+    else std::memcpy(box, s.box, sizeof(s.box));
     if (s.depth > 12) box[6] = 1u;
     if (!box[6]) {
         // cells are 2^(D-T0+1) voxels wide; one voxel of margin on each side
@@ -2640,6 +2663,8 @@ static int build_top(ve_ctx* c, SceneSlot& s) {
             }
         }
     }
+    for (int a = 0; a < 3; a++)
+        if (s.clip_lo[a] != was[a] || s.clip_hi[a] != was[3 + a]) c->scenes_dirty = true;
     return VE_OK;
 }
 
@@ -3904,6 +3929,7 @@ int ve_ctx_destroy(ve_ctx* c) {
     c->hitinfo.release(); c->claim.release(); c->sched_n.release(); c->shade_list.release(); c->scan_tmp.release();
     c->gbuf.release(); c->out_vid.release(); c->out_node.release(); c->out_rgb.release();
     c->out_mapped.release(); c->out_m8.release(); c->path_rgb.release(); c->ray_in.release(); c->ray_out.release();
+    c->edit.release(); c->box.release();
     c->p_sdir.release(); c->p_res.release(); c->res_list.release(); c->em_sort.release(); c->em_sort_tmp.release();
     c->lb_rec.release(); c->lb_keys.release(); c->lb_idx.release(); c->lb_tmp.release();
     c->split_delta.release(); c->d_scenes_split.release(); c->split_cnt.release();
@@ -4294,17 +4320,21 @@ int ve_scene_apply_edits(ve_ctx* c, int32_t id, const uint32_t* slots, const uin
     for (uint64_t i = 0; i < n; i++)
         if (slots[i] >= s.n_words) return fail(VE_ERR_CAPACITY, "scene_apply_edits: slot beyond the uploaded array");
     cudaSetDevice(c->device);
-    if (n) {  // one copy of the (slot, word) lists, one scatter
-        uint32_t* d = nullptr;
-        if (cudaMalloc(&d, n * 8) != cudaSuccess) return fail(VE_ERR_NOMEM, "scene_apply_edits: allocation failed");
-        cudaMemcpyAsync(d, slots, n * 4, cudaMemcpyHostToDevice, c->stream);
-        cudaMemcpyAsync(d + n, words, n * 4, cudaMemcpyHostToDevice, c->stream);
-        k_scatter_words<<<c->num_sms * 4, 256, 0, c->stream>>>(s.nodes, d, d + n, n);
+    uint32_t moved = 0;
+    if (n) {  // the (slot, word) lists, one scatter
+        if (int rc = c->edit.ensure(2 * n + 1)) return rc;
+        uint32_t* d = c->edit.p;
+        cudaMemsetAsync(d, 0, 4, c->stream);
+        cudaMemcpyAsync(d + 1, slots, n * 4, cudaMemcpyHostToDevice, c->stream);
+        cudaMemcpyAsync(d + 1 + n, words, n * 4, cudaMemcpyHostToDevice, c->stream);
+        const uint32_t grid = uint32_t(std::min<uint64_t>((n + 255) / 256, uint64_t(c->num_sms) * 4));
+        k_scatter_words<<<grid, 256, 0, c->stream>>>(s.nodes, d + 1, d + 1 + n, n, d);
+        cudaMemcpyAsync(&moved, d, 4, cudaMemcpyDeviceToHost, c->stream);
         const cudaError_t e = cudaStreamSynchronize(c->stream);
-        cudaFree(d);
+        if (n > kKeptEdits) c->edit.release();
         if (e != cudaSuccess) return fail(VE_ERR_CUDA, std::string("scene_apply_edits: ") + cudaGetErrorString(e));
     }
-    if (int rc = build_top(c, s)) return rc;
+    if (int rc = build_top(c, s, moved != 0u)) return rc;
     if (!(flags & VE_SCENE_KEEP_NORMALS)) {
         int rc = compute_normals(c, s);
         if (rc) return rc;
@@ -4328,14 +4358,16 @@ int ve_scene_refresh(ve_ctx* c, int32_t id, const uint32_t* xyz, uint64_t n, uin
         if (xyz[i] >= L) return fail(VE_ERR_INVALID, "scene_refresh: position outside the scene");
     if (n == 0) return VE_OK;
     cudaSetDevice(c->device);
-    uint32_t* d = nullptr;
-    if (cudaMalloc(&d, n * 12) != cudaSuccess) return fail(VE_ERR_NOMEM, "scene_refresh: allocation failed");
+    if (int rc = c->edit.ensure(3 * n)) return rc;
+    uint32_t* d = c->edit.p;
     cudaMemcpyAsync(d, xyz, n * 12, cudaMemcpyHostToDevice, c->stream);
-    k_refresh<<<c->num_sms * 8, 256, 0, c->stream>>>(s.nodes, s.n_words, s.depth, d, n,
-                                                     (flags & VE_REFRESH_KEEP_CACHE) ? nullptr : s.cache,
-                                                     c->cfg.hash_log2, c->cfg.hash_probes);
+    // one thread per neighbour, 27 per position
+    const uint32_t grid = uint32_t(std::min<uint64_t>((27 * n + 255) / 256, uint64_t(c->num_sms) * 8));
+    k_refresh<<<grid, 256, 0, c->stream>>>(s.nodes, s.n_words, s.depth, d, n,
+                                           (flags & VE_REFRESH_KEEP_CACHE) ? nullptr : s.cache, c->cfg.hash_log2,
+                                           c->cfg.hash_probes);
     const cudaError_t e = cudaStreamSynchronize(c->stream);
-    cudaFree(d);
+    if (n > kKeptEdits) c->edit.release();
     if (e != cudaSuccess) return fail(VE_ERR_CUDA, std::string("scene_refresh: ") + cudaGetErrorString(e));
     return VE_OK;
 }
