@@ -86,7 +86,8 @@ struct Grid {
 
 struct Args {
     const QRec* q;
-    const TRec* tr;            // training only
+    const TRec* tr;            // training only (frames)
+    const float* target;       // training on the caller's rows: 3 floats each, in place of tr
     const uint32_t* count;     // device row count (nullptr: n)
     uint32_t n;                // capacity / row count
     const uint32_t* table;     // fp16 feature pairs, levels x T
@@ -216,8 +217,15 @@ __global__ void __launch_bounds__(128, TRAIN ? 1 : 4) k_nrc_mlp(Args a) {
         bool valid = row < n;
         if (valid) r = a.q[row];
         if (TRAIN && valid) {
-            tr = a.tr[row];
-            valid = tr.valid != 0u;
+            if (a.target) {
+                tr.tr = a.target[3ull * row + 0];
+                tr.tg = a.target[3ull * row + 1];
+                tr.tb = a.target[3ull * row + 2];
+                tr.cell = 0xFFFFFFFFu;
+            } else {
+                tr = a.tr[row];
+                valid = tr.valid != 0u;
+            }
         }
         {
             uint32_t x[32];
@@ -491,10 +499,16 @@ __global__ void __launch_bounds__(256, 4) k_nrc_encode(Args a, uint8_t* __restri
 }
 
 // Output of one inference row: the host-API form stores the prediction.
+// The rows go out as the caller's array has them, 3 floats each, so that the
+// copy to the host is the array itself: with 4-float rows repacked on the host,
+// a call with 262147 rows took 1.78 ms, 0.1 of it on the GPU.
 struct StoreOut {
-    float4* out;
+    float* out;
     __device__ __forceinline__ void operator()(uint8_t*, uint32_t row, bool valid, const float (&y)[3]) const {
-        if (valid) out[row] = make_float4(y[0], y[1], y[2], 0.0f);
+        if (!valid) return;
+        out[3ull * row + 0] = y[0];
+        out[3ull * row + 1] = y[1];
+        out[3ull * row + 2] = y[2];
     }
 };
 

@@ -19,8 +19,7 @@ struct ve_nrc {
     ve::DevBuf<float4> val;  // per validation cell: {mean target, samples}, {mean prediction}
     // host-API staging
     ve::DevBuf<ve::nrc::QRec> q;
-    ve::DevBuf<ve::nrc::TRec> tr;
-    ve::DevBuf<float4> out;
+    ve::DevBuf<float> target, out;  // 3 per row
     // learned-frame buffers: queries (paths terminated at vertex 1) and
     // training samples
     ve::DevBuf<ve::nrc::QRec> fq, fs;
@@ -64,11 +63,12 @@ static Grid make_grid(const ve_nrc_config& cfg) {
     return g;
 }
 
-static int launch_train(ve_nrc* m, cudaStream_t st, const QRec* q, const TRec* tr, const uint32_t* count, uint32_t n,
-                        float inv_norm) {
+static int launch_train(ve_nrc* m, cudaStream_t st, const QRec* q, const TRec* tr, const float* target,
+                        const uint32_t* count, uint32_t n, float inv_norm) {
     Args a{};
     a.q = q;
     a.tr = tr;
+    a.target = target;
     a.count = count;
     a.n = n;
     a.table = m->th.p;
@@ -159,22 +159,10 @@ static int check_status(ve_nrc* m) {
 static int stage_inputs(ve_nrc* m, const ve_nrc_input* in, const float* target, uint32_t n) {
     static_assert(sizeof(ve_nrc_input) == sizeof(QRec), "ve_nrc_input mirrors the device record");
     int rc;
-    if ((rc = m->q.ensure(n)) || (target && (rc = m->tr.ensure(n)))) return rc;
+    if ((rc = m->q.ensure(n)) || (target && (rc = m->target.ensure(3ull * n)))) return rc;
     cudaStream_t st = m->c->stream;
     VE_CUDA(cudaMemcpyAsync(m->q.p, in, sizeof(QRec) * n, cudaMemcpyHostToDevice, st));
-    if (target) {
-        std::vector<TRec> t(n);
-        for (uint32_t i = 0; i < n; i++) {
-            t[i] = TRec{};
-            t[i].tr = target[3 * i];
-            t[i].tg = target[3 * i + 1];
-            t[i].tb = target[3 * i + 2];
-            t[i].valid = 1u;
-            t[i].cell = 0xFFFFFFFFu;
-        }
-        VE_CUDA(cudaMemcpyAsync(m->tr.p, t.data(), sizeof(TRec) * n, cudaMemcpyHostToDevice, st));
-        VE_CUDA(cudaStreamSynchronize(st));
-    }
+    if (target) VE_CUDA(cudaMemcpyAsync(m->target.p, target, sizeof(float) * 3 * n, cudaMemcpyHostToDevice, st));
     return VE_OK;
 }
 
@@ -268,15 +256,13 @@ int ve_nrc_destroy(ve_nrc* m) {
     m->fx.release();
     m->x.release();
     m->th.release();
-    for (auto* b : {&m->w, &m->wm, &m->wv, &m->wg, &m->loss}) b->release();
+    for (auto* b : {&m->w, &m->wm, &m->wv, &m->wg, &m->loss, &m->target, &m->out}) b->release();
     m->val.release();
     m->wimg.release();
     m->adam.release();
     m->status.release();
     m->nvalid.release();
     m->q.release();
-    m->tr.release();
-    m->out.release();
     m->fq.release();
     m->fs.release();
     m->ftr.release();
@@ -346,20 +332,12 @@ int ve_nrc_infer(ve_nrc* m, const ve_nrc_input* in, uint32_t n, float* rgb) {
     if (n == 0) return VE_OK;
     cudaSetDevice(m->c->device);
     int rc;
-    if ((rc = nrc::stage_inputs(m, in, nullptr, n)) || (rc = m->out.ensure(n))) return rc;
+    if ((rc = nrc::stage_inputs(m, in, nullptr, n)) || (rc = m->out.ensure(3ull * n))) return rc;
     cudaStream_t st = m->c->stream;
     if ((rc = m->x.ensure(size_t((n + nrc::kRows - 1) / nrc::kRows) * nrc::kTileBytes))) return rc;
     nrc::launch_infer(m, st, nrc::infer_args(m, m->q.p, nullptr, n), m->x.p, nrc::NoStage{}, nrc::StoreOut{m->out.p});
-    std::vector<float4> o(n);
-    VE_CUDA(cudaMemcpyAsync(o.data(), m->out.p, sizeof(float4) * n, cudaMemcpyDeviceToHost, st));
-    VE_CUDA(cudaStreamSynchronize(st));
-    if ((rc = nrc::check_status(m))) return rc;
-    for (uint32_t i = 0; i < n; i++) {
-        rgb[3 * i] = o[i].x;
-        rgb[3 * i + 1] = o[i].y;
-        rgb[3 * i + 2] = o[i].z;
-    }
-    return VE_OK;
+    VE_CUDA(cudaMemcpyAsync(rgb, m->out.p, sizeof(float) * 3 * n, cudaMemcpyDeviceToHost, st));
+    return nrc::check_status(m);
 }
 
 int ve_nrc_gradients(ve_nrc* m, const ve_nrc_input* in, const float* target, uint32_t n, float* weight_grad,
@@ -370,7 +348,7 @@ int ve_nrc_gradients(ve_nrc* m, const ve_nrc_input* in, const float* target, uin
     cudaStream_t st = m->c->stream;
     int rc;
     if ((rc = nrc::stage_inputs(m, in, target, n)) || (rc = nrc::zero_grads(m, st))) return rc;
-    nrc::launch_train(m, st, m->q.p, m->tr.p, nullptr, n, 1.0f / (3.0f * float(n)));
+    nrc::launch_train(m, st, m->q.p, nullptr, m->target.p, nullptr, n, 1.0f / (3.0f * float(n)));
     float l = 0.0f;
     if (weight_grad)
         VE_CUDA(cudaMemcpyAsync(weight_grad, m->wg.p, sizeof(float) * nrc::kWParams, cudaMemcpyDeviceToHost, st));
@@ -393,7 +371,7 @@ int ve_nrc_train(ve_nrc* m, const ve_nrc_input* in, const float* target, uint32_
     cudaStream_t st = m->c->stream;
     int rc;
     if ((rc = nrc::stage_inputs(m, in, target, n)) || (rc = nrc::zero_grads(m, st))) return rc;
-    nrc::launch_train(m, st, m->q.p, m->tr.p, nullptr, n, 1.0f / (3.0f * float(n)));
+    nrc::launch_train(m, st, m->q.p, nullptr, m->target.p, nullptr, n, 1.0f / (3.0f * float(n)));
     nrc::launch_adam(m, st);
     float l = 0.0f;
     VE_CUDA(cudaMemcpyAsync(&l, m->loss.p, sizeof(float), cudaMemcpyDeviceToHost, st));

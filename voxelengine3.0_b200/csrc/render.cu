@@ -3508,7 +3508,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
             }
             if (train) {
                 nrc::enqueue_zero_grads(nrc, st);
-                nrc::launch_train(nrc, st, nrc->fs.p, nrc->ftr.p, c->counters.p + CNT_NRC_S, a.ns_cap,
+                nrc::launch_train(nrc, st, nrc->fs.p, nrc->ftr.p, nullptr, c->counters.p + CNT_NRC_S, a.ns_cap,
                                   1.0f / (3.0f * float(a.ns_cap)));
                 nrc::launch_adam(nrc, st);
                 launches += 4;
