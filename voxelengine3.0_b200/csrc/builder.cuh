@@ -33,12 +33,19 @@ __device__ __forceinline__ uint64_t morton(uint32_t x, uint32_t y, uint32_t z, u
     return k;
 }
 
-__global__ void k_keys(const uint32_t* __restrict__ xyzm, uint64_t n, uint32_t D, uint64_t* __restrict__ keys,
-                       uint32_t* __restrict__ idx) {
+// Sets bit 0 of *bad for a voxel outside the cube, bit 1 for a material other
+// than 1..127 (its key is then that of the low bits; the caller stops).
+__global__ void k_keys(const uint4* __restrict__ xyzm, uint64_t n, uint32_t D, uint64_t* __restrict__ keys,
+                       uint32_t* __restrict__ idx, uint32_t* bad) {
+    uint32_t wrong = 0;
     for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
-        keys[i] = morton(xyzm[4 * i], xyzm[4 * i + 1], xyzm[4 * i + 2], D);
+        const uint4 v = xyzm[i];
+        wrong |= ((v.x | v.y | v.z) >> D) != 0u ? 1u : 0u;
+        wrong |= v.w - 1u > 126u ? 2u : 0u;
+        keys[i] = morton(v.x, v.y, v.z, D);
         idx[i] = uint32_t(i);
     }
+    if (wrong) atomicOr(bad, wrong);
 }
 
 // keep the last voxel of each run of equal keys

@@ -2226,8 +2226,13 @@ constexpr uint64_t kKeptEdits = 1u << 20;
 // rays per piece of a batch (ve_raycast_batch); a smaller batch goes whole
 constexpr uint64_t kRayPiece = 1u << 17;
 
+// bytes of freed build and normal-pass scratch a context keeps for its next
+// build (the pool is emptied with the context)
+constexpr uint64_t kScratchKept = 512ull << 20;
+
 struct ve_ctx {
     int device = 0;
+    cudaMemPool_t scratch = nullptr;  // stream-ordered scratch of scene builds and normal passes
     int num_sms = 148;
     cudaStream_t stream = nullptr;
     ve_renderer_config cfg{};
@@ -2670,25 +2675,54 @@ static int build_top(ve_ctx* c, SceneSlot& s, bool rebuild = true) {
     return VE_OK;
 }
 
+// Stream-ordered device scratch, freed on every exit path: a build makes about
+// 50 allocations, which with cudaMalloc / cudaFree (each one stops the device)
+// took 20 ms of a 4 M-voxel build.
+struct Scratch {
+    ve_ctx* c;
+    std::vector<void*> ptrs;
+    explicit Scratch(ve_ctx* ctx) : c(ctx) {}
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+    ~Scratch() {
+        for (void* p : ptrs) cudaFreeAsync(p, c->stream);
+    }
+    template <typename T>
+    T* alloc(size_t n) {
+        void* p = nullptr;
+        const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
+        if (!c->scratch) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = c->device;
+            uint64_t keep = kScratchKept;
+            if (cudaMemPoolCreate(&c->scratch, &props) != cudaSuccess ||
+                cudaMemPoolSetAttribute(c->scratch, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+        }
+        if (cudaMallocFromPoolAsync(&p, bytes, c->scratch, c->stream) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        ptrs.push_back(p);
+        return static_cast<T*>(p);
+    }
+};
+
 static int compute_normals(ve_ctx* c, SceneSlot& s) {
     const uint32_t D = s.depth;
     if (D < 1 || D > 11) return VE_OK;
     const uint64_t cap = std::max<uint64_t>(s.n_words, 16);
-    unsigned long long *fa = nullptr, *fb = nullptr;
-    uint32_t* cnt = nullptr;
-    uint32_t* occ = nullptr;
     const uint64_t occ_words = ((1ull << (3 * D)) + 31) / 32;
-    auto cleanup = [&]() {
-        if (fa) cudaFree(fa);
-        if (fb) cudaFree(fb);
-        if (cnt) cudaFree(cnt);
-        if (occ) cudaFree(occ);
-    };
-    if (cudaMalloc(&fa, cap * 8) != cudaSuccess || cudaMalloc(&fb, cap * 8) != cudaSuccess ||
-        cudaMalloc(&cnt, 64 * 4) != cudaSuccess || cudaMalloc(&occ, occ_words * 4) != cudaSuccess) {
-        cleanup();
-        return fail(VE_ERR_NOMEM, "normal pass: device allocation failed");
-    }
+    Scratch scratch(c);
+    unsigned long long* fa = scratch.alloc<unsigned long long>(cap);
+    unsigned long long* fb = scratch.alloc<unsigned long long>(cap);
+    uint32_t* cnt = scratch.alloc<uint32_t>(64);
+    uint32_t* occ = scratch.alloc<uint32_t>(occ_words);
+    if (!fa || !fb || !cnt || !occ) return fail(VE_ERR_NOMEM, "normal pass: device allocation failed");
     cudaMemsetAsync(cnt, 0, 64 * 4, c->stream);
     cudaMemsetAsync(occ, 0, occ_words * 4, c->stream);
     const unsigned long long root = 0ull;  // slot 0, origin (0,0,0), level 0
@@ -2708,7 +2742,6 @@ static int compute_normals(ve_ctx* c, SceneSlot& s) {
     if (s.normal_radius == 0u) {
         k_leaf_pass<<<grid, 256, 0, c->stream>>>(s.nodes, s.n_words, D, in, lc, occ, 1, uint32_t(cap));
         cudaError_t e = cudaStreamSynchronize(c->stream);
-        cleanup();
         if (e != cudaSuccess) return fail(VE_ERR_CUDA, std::string("normal pass: ") + cudaGetErrorString(e));
         if (s.ntab) {  // back from the ball mode
             cudaFree(s.ntab);
@@ -2720,29 +2753,21 @@ static int compute_normals(ve_ctx* c, SceneSlot& s) {
     }
     // the reference's ball mode: a code per leaf, then the sorted table of
     // distinct codes, and every leaf's index into it
-    if (s.n_words > uint64_t(INT32_MAX)) {
-        cleanup();
-        return fail(VE_ERR_CAPACITY, "normal pass (ball): more than 2^31 words");
-    }
+    if (s.n_words > uint64_t(INT32_MAX)) return fail(VE_ERR_CAPACITY, "normal pass (ball): more than 2^31 words");
     const int nw = int(s.n_words);
     uint32_t *codes = nullptr, *sel = nullptr, *table = nullptr, *nsel = nullptr;
-    void* tmp = nullptr;
-    auto cleanup2 = [&]() {
-        cleanup();
-        for (void* p : {(void*)codes, (void*)sel, (void*)table, (void*)nsel, tmp})
-            if (p) cudaFree(p);
-    };
     size_t b_sel = 0, b_sort = 0, b_uniq = 0;
     cub::DeviceSelect::If(nullptr, b_sel, codes, sel, nsel, nw, NonZero(), c->stream);
     cub::DeviceRadixSort::SortKeys(nullptr, b_sort, sel, table, nw, 2, 32, c->stream);
     cub::DeviceSelect::Unique(nullptr, b_uniq, table, sel, nsel + 1, nw, c->stream);
     const size_t b_tmp = std::max(b_sel, std::max(b_sort, b_uniq));
-    if (cudaMalloc(&codes, size_t(nw) * 4) != cudaSuccess || cudaMalloc(&sel, size_t(nw) * 4) != cudaSuccess ||
-        cudaMalloc(&table, size_t(nw) * 4) != cudaSuccess || cudaMalloc(&nsel, 2 * 4) != cudaSuccess ||
-        cudaMalloc(&tmp, std::max<size_t>(b_tmp, 16)) != cudaSuccess) {
-        cleanup2();
+    codes = scratch.alloc<uint32_t>(size_t(nw));
+    sel = scratch.alloc<uint32_t>(size_t(nw));
+    table = scratch.alloc<uint32_t>(size_t(nw));
+    nsel = scratch.alloc<uint32_t>(2);
+    void* tmp = scratch.alloc<uint8_t>(std::max<size_t>(b_tmp, 16));
+    if (!codes || !sel || !table || !nsel || !tmp)
         return fail(VE_ERR_NOMEM, "normal pass (ball): device allocation failed");
-    }
     cudaMemsetAsync(codes, 0, size_t(nw) * 4, c->stream);
     k_ball_codes<<<grid, 256, 0, c->stream>>>(s.nodes, s.n_words, D, in, lc, occ, int(s.normal_radius), codes,
                                               uint32_t(cap));
@@ -2759,17 +2784,13 @@ static int compute_normals(ve_ctx* c, SceneSlot& s) {
         cudaMemcpyAsync(&h_n[1], nsel + 1, 4, cudaMemcpyDeviceToHost, c->stream);
         e = cudaStreamSynchronize(c->stream);
     }
-    if (e != cudaSuccess) {
-        cleanup2();
-        return fail(VE_ERR_CUDA, std::string("normal pass (ball): ") + cudaGetErrorString(e));
-    }
+    if (e != cudaSuccess) return fail(VE_ERR_CUDA, std::string("normal pass (ball): ") + cudaGetErrorString(e));
     if (s.ntab) cudaFree(s.ntab);
     s.ntab = nullptr;
     s.n_ntab = 0;
     if (h_n[1] > 0u) {
         if (cudaMalloc(&s.ntab, size_t(h_n[1]) * sizeof(float4)) != cudaSuccess) {
             s.ntab = nullptr;
-            cleanup2();
             return fail(VE_ERR_NOMEM, "normal pass (ball): table allocation failed");
         }
         s.n_ntab = h_n[1];
@@ -2777,7 +2798,6 @@ static int compute_normals(ve_ctx* c, SceneSlot& s) {
         k_ball_apply<<<grid, 256, 0, c->stream>>>(s.nodes, s.n_words, codes, sel, h_n[1]);
     }
     e = cudaStreamSynchronize(c->stream);
-    cleanup2();
     c->scenes_dirty = true;
     if (e != cudaSuccess) return fail(VE_ERR_CUDA, std::string("normal pass (ball): ") + cudaGetErrorString(e));
     return VE_OK;
@@ -3975,6 +3995,7 @@ int ve_ctx_destroy(ve_ctx* c) {
             if (e) cudaEventDestroy(e);
     for (auto& g : c->graphs)
         if (g.exec) cudaGraphExecDestroy(g.exec);
+    if (c->scratch) cudaMemPoolDestroy(c->scratch);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return VE_OK;
@@ -4024,21 +4045,6 @@ int ve_ctx_synchronize(ve_ctx* c) {
 
 namespace ve {
 
-// Device scratch of the bulk builder, freed on every exit path.
-struct BuildScratch {
-    std::vector<void*> ptrs;
-    ~BuildScratch() {
-        for (void* p : ptrs) cudaFree(p);
-    }
-    template <typename T>
-    T* alloc(size_t n) {
-        void* p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) return nullptr;
-        ptrs.push_back(p);
-        return static_cast<T*>(p);
-    }
-};
-
 #define VE_BUILD_ALLOC(ptr, T, n)                                    \
     T* ptr = scratch.alloc<T>(n);                                   \
     if (!ptr) return fail(VE_ERR_NOMEM, "scene_build: device allocation failed")
@@ -4046,12 +4052,13 @@ struct BuildScratch {
 // Node words of OctreeCPU::insert (all voxels) + Octree::set, built on the
 // device (builder.cuh).  `xyzm` is a device array of n (x, y, z, material).
 // On success *words is a cudaMalloc'd array of *n_words words placed 7 words
-// into the allocation (*alloc), like an uploaded scene.
+// into the allocation (*alloc), like an uploaded scene.  Voxels outside the
+// cube or with a material other than 1..127 are found by the key pass.
 static int build_scene_words(ve_ctx* c, const uint32_t* xyzm, uint64_t n, uint32_t D, void** alloc,
                              uint32_t** words, uint64_t* n_words) {
     using namespace build;
     cudaStream_t st = c->stream;
-    BuildScratch scratch;
+    Scratch scratch(c);
     const int grid = c->num_sms * 8;
     auto run_cub = [&](auto&& fn) -> int {  // size query, then the run
         size_t bytes = 0;
@@ -4079,8 +4086,10 @@ static int build_scene_words(ve_ctx* c, const uint32_t* xyzm, uint64_t n, uint32
     VE_BUILD_ALLOC(idx, uint32_t, n);
     VE_BUILD_ALLOC(idx_s, uint32_t, n);
     VE_BUILD_ALLOC(flag, uint8_t, n);
-    VE_BUILD_ALLOC(nsel, uint64_t, 1);
-    k_keys<<<grid, 256, 0, st>>>(xyzm, n, D, keys, idx);
+    VE_BUILD_ALLOC(nsel, uint64_t, 2);
+    uint32_t* bad = reinterpret_cast<uint32_t*>(nsel + 1);
+    VE_CUDA(cudaMemsetAsync(bad, 0, 8, st));
+    k_keys<<<grid, 256, 0, st>>>(reinterpret_cast<const uint4*>(xyzm), n, D, keys, idx, bad);
     if ((rc = run_cub([&](void* t, size_t& b) {
              return cub::DeviceRadixSort::SortPairs(t, b, keys, keys_s, idx, idx_s, n, 0, int(3 * D), st);
          })))
@@ -4095,9 +4104,12 @@ static int build_scene_words(ve_ctx* c, const uint32_t* xyzm, uint64_t n, uint32
              return cub::DeviceSelect::Flagged(t, b, idx_s, flag, leaf_idx, nsel, n, st);
          })))
         return rc;
-    uint64_t nu = 0;
-    VE_CUDA(cudaMemcpyAsync(&nu, nsel, 8, cudaMemcpyDeviceToHost, st));
+    uint64_t got[2] = {0, 0};
+    VE_CUDA(cudaMemcpyAsync(got, nsel, 16, cudaMemcpyDeviceToHost, st));
     VE_CUDA(cudaStreamSynchronize(st));
+    const uint64_t nu = got[0];
+    if (uint32_t(got[1]) & 1u) return fail(VE_ERR_INVALID, "scene_build: voxel outside the 2^depth cube");
+    if (uint32_t(got[1]) & 2u) return fail(VE_ERR_INVALID, "scene_build: materials are 1..127");
     if (nu == 0) return empty_scene();
     VE_BUILD_ALLOC(leaf_mat, uint32_t, nu);
     k_gather_material<<<grid, 256, 0, st>>>(xyzm, leaf_idx, nu, leaf_mat);
@@ -4190,24 +4202,21 @@ int ve_scene_build(ve_ctx* c, const uint32_t* xyzm, uint64_t n, uint32_t depth, 
     if (!c || (!xyzm && n) || !scene_id) return fail(VE_ERR_INVALID, "scene_build: null argument");
     if (depth < 1 || depth > 16) return fail(VE_ERR_INVALID, "scene_build: depth must be in [1, 16]");
     if (n >= (1ull << 32)) return fail(VE_ERR_CAPACITY, "scene_build: at most 2^32 - 1 voxels");
-    const uint64_t L = 1ull << depth;
-    for (uint64_t i = 0; i < n; i++) {
-        if (xyzm[4 * i] >= L || xyzm[4 * i + 1] >= L || xyzm[4 * i + 2] >= L)
-            return fail(VE_ERR_INVALID, "scene_build: voxel outside the 2^depth cube");
-        if (xyzm[4 * i + 3] == 0u || xyzm[4 * i + 3] > 127u)
-            return fail(VE_ERR_INVALID, "scene_build: materials are 1..127");
-    }
     cudaSetDevice(c->device);
-    uint32_t* d_in = nullptr;
-    if (cudaMalloc(&d_in, std::max<uint64_t>(n, 1) * 16) != cudaSuccess)
-        return fail(VE_ERR_NOMEM, "scene_build: device allocation failed");
-    if (n) VE_CUDA(cudaMemcpyAsync(d_in, xyzm, n * 16, cudaMemcpyHostToDevice, c->stream));
     SceneSlot s;
     s.depth = depth;
-    int rc = build_scene_words(c, d_in, n, depth, &s.alloc, &s.nodes, &s.n_words);
-    cudaStreamSynchronize(c->stream);
-    cudaFree(d_in);
-    if (rc) return rc;
+    {
+        Scratch in(c);
+        uint32_t* d_in = in.alloc<uint32_t>(4 * n);
+        if (!d_in) return fail(VE_ERR_NOMEM, "scene_build: device allocation failed");
+        if (n) VE_CUDA(cudaMemcpyAsync(d_in, xyzm, n * 16, cudaMemcpyHostToDevice, c->stream));
+        const int rc = build_scene_words(c, d_in, n, depth, &s.alloc, &s.nodes, &s.n_words);
+        if (rc) {
+            cudaStreamSynchronize(c->stream);
+            return rc;
+        }
+    }
+    int rc = VE_OK;
     const size_t cache_bytes = sizeof(CacheEntry) << c->cfg.hash_log2;
     if (cudaMalloc(&s.cache, cache_bytes) != cudaSuccess) {
         cudaFree(s.alloc);
