@@ -486,7 +486,7 @@ int ve_server_get_stats(ve_server* s, ve_server_stats* out) {
     uint64_t scene_bytes = 0;
     for (const auto& sc : s->c->scenes)
         if (sc.live)
-            scene_bytes += (sc.n_words + kNodePad) * 4 + (sizeof(CacheEntry) << s->c->cfg.hash_log2) +
+            scene_bytes += (sc.n_words + kNodePad) * 4 + sizeof(CacheEntry) * cache_entries(s->c->cfg.hash_log2) +
                            4ull * top_words(sc.top_level);
     out->scene_bytes = scene_bytes;
     out->rays = s->rays;
