@@ -1640,32 +1640,41 @@ __global__ void __launch_bounds__(256, 4) k_sched_emit(FrameArgs a) {
 // ---------------------------------------------------------------------------
 // End-of-frame commits of emissive frames.
 // ---------------------------------------------------------------------------
-// Registry: sort keys = the staged lights' vids (unused slots ~0), values =
-// staging indices.
-__global__ void __launch_bounds__(256) k_em_keys(const DevScene* scenes, uint32_t sc, uint32_t* keys, uint32_t* vals) {
-    const DevScene S = scenes[sc];
-    constexpr uint32_t cap = 1u << kEmClaimLog2;
-    const uint32_t n = min(S.em_state[1], cap);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += gridDim.x * blockDim.x) {
-        keys[i] = i < n ? S.em_stage[i].vid : 0xFFFFFFFFu;
-        vals[i] = i;
-    }
-}
-// ... the staged lights in vid order fill the registry's free records (one
-// block: every thread reads the counts before thread 0 updates them).
-__global__ void __launch_bounds__(1024) k_em_append(const DevScene* scenes, uint32_t sc, const uint32_t* order,
-                                                    unsigned long long* stats) {
+// The staged lights in vid order fill the registry's free records: a light's
+// place is the number of staged vids below its own (vids are distinct), counted
+// from shared memory.  After its first frames a scene stages few lights or none,
+// and the kernel ends at once; a radix sort of all 2^17 staging slots took
+// 42 us of every frame.  (4096 new lights: 5 us; 2^17, which only a first frame can
+// have: about 1 ms, once.)
+__global__ void __launch_bounds__(256) k_em_rank(const DevScene* scenes, uint32_t sc) {
+    __shared__ uint32_t vids[1024];
     const DevScene S = scenes[sc];
     const uint32_t count = min(S.em_state[0], kEmCapacity);
     const uint32_t n = min(S.em_state[1], 1u << kEmClaimLog2);
     const uint32_t add = min(n, kEmCapacity - count);
-    for (uint32_t i = threadIdx.x; i < add; i += blockDim.x) S.em_list[count + i] = S.em_stage[order[i]];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        S.em_state[0] = count + add;
-        S.em_state[1] = 0u;
-        atomicAdd(&stats[ST_EM_LIGHTS], (unsigned long long)(count + add));
+    if (add == 0u) return;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+        const uint32_t i = base + threadIdx.x;
+        const uint32_t vid = i < n ? S.em_stage[i].vid : 0u;
+        uint32_t rank = 0;
+        for (uint32_t t = 0; t < n; t += 1024u) {
+            __syncthreads();
+            for (uint32_t k = threadIdx.x; k < 1024u; k += blockDim.x)
+                vids[k] = t + k < n ? S.em_stage[t + k].vid : 0xFFFFFFFFu;
+            __syncthreads();
+#pragma unroll 8
+            for (uint32_t k = 0; k < 1024u; k++) rank += vids[k] < vid ? 1u : 0u;
+        }
+        if (i < n && rank < add) S.em_list[count + rank] = S.em_stage[i];
     }
+}
+__global__ void k_em_append(const DevScene* scenes, uint32_t sc, unsigned long long* stats) {
+    const DevScene S = scenes[sc];
+    const uint32_t count = min(S.em_state[0], kEmCapacity);
+    const uint32_t add = min(min(S.em_state[1], 1u << kEmClaimLog2), kEmCapacity - count);
+    S.em_state[0] = count + add;
+    S.em_state[1] = 0u;
+    atomicAdd(&stats[ST_EM_LIGHTS], (unsigned long long)(count + add));
 }
 // Reservoirs: each voxel keeps the reservoir of its winning path (the
 // largest slot among the frame's bounce-0 paths on it).
@@ -2327,8 +2336,6 @@ struct ve_ctx {
     ve::DevBuf<float4> p_sdir;          // emissive batches: NEE shadow directions + light vid
     ve::DevBuf<ve::PathRes> p_res;      // emissive batches: bounce-0 reservoirs until the commit
     ve::DevBuf<uint32_t> res_list;      // ... and the paths that hold one
-    ve::DevBuf<uint32_t> em_sort;       // registry commit: vid keys / staging indices, 2 x 2 x 2^17
-    ve::DevBuf<uint8_t> em_sort_tmp;    // ... CUB radix-sort scratch
     ve::DevBuf<ve::LbRec> lb_rec;        // lBuffer frames: deposits at their path slots
     ve::DevBuf<uint32_t> lb_keys;        // ... their rows (0: none), 2 x paths (sort in, out)
     ve::DevBuf<uint32_t> lb_idx;         // ... path slots 0..n-1 (sort values in), order (out), row bounds
@@ -3304,7 +3311,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         if (old != c->path_rgb.p) c->gen++;
     }
     // emissive lights: the scenes' registries and reservoir tables, the
-    // per-path NEE records and the registry commit's sort buffers
+    // per-path NEE records
     // the trace's FLAT instance: every view's scene has a top table reaching
     // its leaves (depth 3..10)
     // ... and its one-scene form: all of them show the same scene
@@ -3315,7 +3322,6 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         flat = flat && sc.top_level != 0u && sc.top_level == sc.depth;
     }
     std::vector<int> em_scenes;
-    size_t em_sort_bytes = 0;
     if (flags & VE_FRAME_EMISSIVE) {
         for (uint32_t i = 0; i < nv; i++) {
             if (!(views[i].frame.flags & VE_FRAME_EMISSIVE)) continue;
@@ -3323,15 +3329,11 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
             if (std::find(em_scenes.begin(), em_scenes.end(), sc) == em_scenes.end()) em_scenes.push_back(sc);
             if ((rc = ensure_emissive(c, c->scenes[sc]))) return rc;
         }
-        constexpr int cap = 1 << kEmClaimLog2;
-        cub::DeviceRadixSort::SortPairs(nullptr, em_sort_bytes, (const uint32_t*)nullptr, (uint32_t*)nullptr,
-                                        (const uint32_t*)nullptr, (uint32_t*)nullptr, cap, 0, 32, c->stream);
-        const void* before[] = {c->p_sdir.p, c->p_res.p, c->res_list.p, c->em_sort.p, c->em_sort_tmp.p};
-        if ((rc = c->p_sdir.ensure(paths)) || (rc = c->p_res.ensure(paths)) || (rc = c->res_list.ensure(paths)) ||
-            (rc = c->em_sort.ensure(4ull * cap)) || (rc = c->em_sort_tmp.ensure(em_sort_bytes)))
+        const void* before[] = {c->p_sdir.p, c->p_res.p, c->res_list.p};
+        if ((rc = c->p_sdir.ensure(paths)) || (rc = c->p_res.ensure(paths)) || (rc = c->res_list.ensure(paths)))
             return rc;
-        const void* after[] = {c->p_sdir.p, c->p_res.p, c->res_list.p, c->em_sort.p, c->em_sort_tmp.p};
-        for (int i = 0; i < 5; i++)
+        const void* after[] = {c->p_sdir.p, c->p_res.p, c->res_list.p};
+        for (int i = 0; i < 3; i++)
             if (before[i] != after[i]) c->gen++;
     }
     size_t lb_sort_bytes = 0;
@@ -3596,17 +3598,10 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
             launches++;
         }
         if (flags & VE_FRAME_EMISSIVE) {  // this frame's lights and reservoirs, for the next frame
-            constexpr int cap = 1 << kEmClaimLog2;
-            uint32_t* kin = c->em_sort.p;
-            uint32_t* kout = kin + cap;
-            uint32_t* vin = kin + 2 * cap;
-            uint32_t* vout = kin + 3 * cap;
             for (int sc : em_scenes) {
-                k_em_keys<<<c->num_sms * 4, 256, 0, st>>>(a.scenes, uint32_t(sc), kin, vin);
-                size_t b = em_sort_bytes;
-                cub::DeviceRadixSort::SortPairs(c->em_sort_tmp.p, b, kin, kout, vin, vout, cap, 0, 32, st);
-                k_em_append<<<1, 1024, 0, st>>>(a.scenes, uint32_t(sc), vout, c->stats.p);
-                launches += 3;
+                k_em_rank<<<c->num_sms * 2, 256, 0, st>>>(a.scenes, uint32_t(sc));
+                k_em_append<<<1, 1, 0, st>>>(a.scenes, uint32_t(sc), c->stats.p);
+                launches += 2;
             }
             k_res_commit<<<c->num_sms * 4, 256, 0, st>>>(a);
             launches++;
@@ -3986,7 +3981,7 @@ int ve_ctx_destroy(ve_ctx* c) {
     c->gbuf.release(); c->out_vid.release(); c->out_node.release(); c->out_rgb.release();
     c->out_mapped.release(); c->out_m8.release(); c->path_rgb.release(); c->ray_in.release(); c->ray_out.release();
     c->edit.release(); c->box.release();
-    c->p_sdir.release(); c->p_res.release(); c->res_list.release(); c->em_sort.release(); c->em_sort_tmp.release();
+    c->p_sdir.release(); c->p_res.release(); c->res_list.release();
     c->lb_rec.release(); c->lb_keys.release(); c->lb_idx.release(); c->lb_tmp.release();
     c->split_delta.release(); c->d_scenes_split.release(); c->split_cnt.release();
     if (c->copy_stream) {
