@@ -221,8 +221,7 @@ __device__ __forceinline__ bool dda_step(Dda& s, const uint32_t* __restrict__ no
 //     a rising axis (low 22 bits all ones) and of -1.5 * 2^23 for a falling one
 //     (all zeros), ((b ^ c) & ~m) ^ c is the cell's last coordinate or its
 //     first one (m = cell size - 1), and adding c as a float gives the plane.
-//   * The cell is its table entry, whose mask is compared with the changed bits
-//     of the position: no level, no leading-zero count.
+//   * The cell is its table entry: no level, no leading-zero count.
 //   * min/max of three operands are one instruction each.  They return what
 //     the glm selects of dda_step return: inside the volume no exit distance
 //     is NaN (an axis with 1/d = +-inf has a non-zero numerator of its sign),
@@ -337,7 +336,10 @@ __device__ __forceinline__ uint32_t flat_first(FlatRay& s, const FlatScene& w) {
 // while the leaf word is on its way: a step waits for one load, not two (1080p
 // depth-10 frame: trace 0.594 -> 0.545 ms, primary 0.351 -> 0.324; 256x256
 // depth 7: 0.047 -> 0.042 and 0.0345 -> 0.0273).  A ray that hits has loaded
-// one entry in vain.
+// one entry in vain.  The entry is loaded at every step, also inside the leaf
+// block or cell it was loaded for: the test that spared those (cached) loads
+// cost more (2160p 8 spp frame: trace 2.93 -> 2.77 ms without it, 1080p 0.520 ->
+// 0.508).
 // WORD: a hit leaves the leaf's word in ent, else its slot.  CLIP as in
 // dda_step.
 template <bool WORD, bool CLIP>
@@ -352,15 +354,13 @@ __device__ __forceinline__ uint32_t flat_step(FlatRay& s, const FlatScene& w) {
                 flat_exit(s.bz, m, s.o.z, s.inv.z));
     uint32_t bx, by, bz;
     const bool in = flat_at<CLIP>(s, w, bx, by, bz);
-    const uint32_t xd = (bx ^ s.bx) | (by ^ s.by) | (bz ^ s.bz);
-    uint32_t ent = s.ent;
-    if (in && xd > (m | 1u)) ent = flat_entry(w, bx, by, bz);  // neither this cell nor its leaf block
-    if (raw & 254u) {
-        s.ent = WORD ? raw : off;
-        return kHit;
+    uint32_t ent = 0u;
+    if (in) ent = flat_entry(w, bx, by, bz);
+    if ((raw & 254u) != 0u || !in || s.left == 0u) {
+        const bool hit = (raw & 254u) != 0u;
+        if (hit) s.ent = WORD ? raw : off;
+        return hit ? kHit : in ? kTimeout : kEscaped;
     }
-    if (!in) return kEscaped;
-    if (s.left == 0u) return kTimeout;
     s.left--;
     s.bx = bx; s.by = by; s.bz = bz;
     s.ent = ent;
