@@ -2267,6 +2267,7 @@ constexpr uint64_t kRayPiece = 1u << 17;
 // bytes of freed build and normal-pass scratch a context keeps for its next
 // build (the pool is emptied with the context)
 constexpr uint64_t kScratchKept = 512ull << 20;
+constexpr size_t kScratchLarge = 128u << 20;  // larger pieces are allocated and freed each time
 
 struct ve_ctx {
     int device = 0;
@@ -2716,17 +2717,26 @@ static int build_top(ve_ctx* c, SceneSlot& s, bool rebuild = true) {
 // took 20 ms of a 4 M-voxel build.
 struct Scratch {
     ve_ctx* c;
-    std::vector<void*> ptrs;
+    std::vector<void*> ptrs, large;
     explicit Scratch(ve_ctx* ctx) : c(ctx) {}
     Scratch(const Scratch&) = delete;
     Scratch& operator=(const Scratch&) = delete;
     ~Scratch() {
         for (void* p : ptrs) cudaFreeAsync(p, c->stream);
+        for (void* p : large) cudaFree(p);
     }
     template <typename T>
     T* alloc(size_t n) {
         void* p = nullptr;
         const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
+        if (bytes > kScratchLarge) {  // would not be kept, and a pool grows slower than cudaMalloc
+            if (cudaMalloc(&p, bytes) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            large.push_back(p);
+            return static_cast<T*>(p);
+        }
         if (!c->scratch) {
             cudaMemPoolProps props{};
             props.allocType = cudaMemAllocationTypePinned;
