@@ -223,6 +223,7 @@ struct FrameArgs {
     uint2* shade_list;      // {vid, pixel} per path
     uint32_t shade_cap;
     float* rank;            // the scene's {t_high, t_mid, histogram[256]} (thresholds from the previous frame)
+    bool early_ids;         // the primary pass writes out_vid / out_node (kEarlyIds), not the AvgPass
     FlatScene one;          // the batch's scene when all its views share one whose table reaches the leaves
 };
 
@@ -1210,6 +1211,10 @@ __global__ void __launch_bounds__(256, 4) k_primary(FrameArgs a) {
         const uint32_t pix = py * v.W + px;
         a.gbuf[v.pix_base + pix] = make_uint4(h.checks, h.status == kHit ? h.material : 0u,
                                               h.status == kHit ? h.id : 0u, vid);
+        if (a.early_ids) {  // the id images, so that their copy can start now
+            a.out_vid[v.pix_base + pix] = vid;
+            a.out_node[v.pix_base + pix] = h.status == kHit ? h.id : 0u;
+        }
         if (v.flags & VE_FRAME_SCHEDULED)  // paths come from the shade list: keep the hit
             a.hitinfo[v.pix_base + pix] = make_uint4(word, h.x | (h.y << 16), h.z | (h.material << 16), 0u);
     }
@@ -1966,8 +1971,10 @@ __global__ void __launch_bounds__(256) k_resolve(FrameArgs a) {
             break;
         }
     }
-    if (a.out_vid) a.out_vid[gp] = vid;
-    if (a.out_node) a.out_node[gp] = node;
+    if (!a.early_ids) {
+        if (a.out_vid) a.out_vid[gp] = vid;
+        if (a.out_node) a.out_node[gp] = node;
+    }
     if (a.out_rgb) {
         a.out_rgb[3ull * gp + 0] = col.x;
         a.out_rgb[3ull * gp + 1] = col.y;
@@ -3136,6 +3143,19 @@ static void fill_view(DevView& d, const ve_view& v) {
     set_rows(d, f, (f.flags & VE_FRAME_SPLIT) != 0);
 }
 
+// Bytes of id images from which they leave early.  Below, the second graph
+// launch costs what the copy would.
+constexpr uint64_t kEarlyIds = 2ull << 20;
+
+static bool pinned_host(const void* p) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeHost;
+}
+
 static int ensure_copy_stream(ve_ctx* c) {
     if (!c->copy_stream) {
         if (cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
@@ -3238,10 +3258,26 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
     // VE_CFG_PIPELINE: plain frames whose primary pass takes no path to a
     // deposit (every view has a bounce) alternate between the two frame sets;
     // anything else runs on the main stream after the second set's frames
-    const bool pipe = (c->cfg.flags & VE_CFG_PIPELINE) && !split && min_b >= 1 && !c->scenes_dirty &&
-                      !(flags & (VE_FRAME_TIMING | VE_FRAME_COUNT_FETCH | VE_FRAME_PATH_RGB | VE_FRAME_LEARNED |
-                                 VE_FRAME_TERMINATE_HASH | VE_FRAME_TRAIN | VE_FRAME_SCHEDULED | VE_FRAME_EMISSIVE |
-                                 VE_FRAME_LBUFFER));
+    const bool plain = !split && min_b >= 1 &&
+                       !(flags & (VE_FRAME_TIMING | VE_FRAME_COUNT_FETCH | VE_FRAME_PATH_RGB | VE_FRAME_LEARNED |
+                                  VE_FRAME_TERMINATE_HASH | VE_FRAME_TRAIN | VE_FRAME_SCHEDULED | VE_FRAME_EMISSIVE |
+                                  VE_FRAME_LBUFFER));
+    const bool pipe = (c->cfg.flags & VE_CFG_PIPELINE) && plain && !c->scenes_dirty;
+    // Large voxel-id and hit-node images of a plain frame are complete after its
+    // primary pass: that pass writes them and they are copied out while the
+    // bounces run (the copy of 12 mixed views' ids is a seventh of the call).
+    // Pinned destinations only: a pageable copy would hold up the launches.
+    uint64_t early_bytes = 0;
+    if (plain && outs && !(flags & VE_FRAME_ASYNC_OUTPUTS)) {
+        for (uint32_t i = 0; i < nv; i++) {
+            const uint64_t np = uint64_t(views[i].frame.width) * views[i].frame.height;
+            early_bytes += (outs[i].voxel_id ? 4 * np : 0) + (outs[i].hit_node ? 4 * np : 0);
+        }
+        for (uint32_t i = 0; early_bytes >= kEarlyIds && i < nv; i++)
+            if ((outs[i].voxel_id && !pinned_host(outs[i].voxel_id)) || (outs[i].hit_node && !pinned_host(outs[i].hit_node)))
+                early_bytes = 0;
+    }
+    const bool early = early_bytes >= kEarlyIds;
     if (!pipe) join_alt(c);
     const int set = pipe ? c->pipe_next : 0;
     if (pipe) {
@@ -3498,6 +3534,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         a.p_res = c->p_res.p;
         a.res_list = c->res_list.p;
     }
+    a.early_ids = early;
     one = one && flat;
     if (one) {
         const SceneSlot& sc = c->scenes[views[0].scene_id];
@@ -3620,7 +3657,9 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         k_accum_stats<<<1, 32, 0, st>>>(c->stats.p, c->totals.p);
         launches++;
     };
-    // this frame's resolve overwrites an image set whose copy may be pending
+    if (early)
+        if (int e = ensure_copy_stream(c)) return e;
+    // this frame overwrites an image set whose copy may be pending
     if (c->copy_stream) VE_CUDA(cudaStreamWaitEvent(st, c->copy_done[parity], 0));
     const bool use_graph = !timing && !(c->cfg.flags & VE_CFG_NO_GRAPHS);
     // one part of the frame: enqueued directly, or as the replay of its
@@ -3644,7 +3683,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         }
         for (int sc : em_scenes) key.push_back((1ull << 62) | uint64_t(uint32_t(sc)));
         key.push_back((1ull << 61) | uint64_t(parity));
-        key.push_back((1ull << 59) | uint64_t(flat));
+        key.push_back((1ull << 59) | (uint64_t(early) << 1) | uint64_t(flat));
         if (one) key.push_back((1ull << 58) | uint64_t(uint32_t(views[0].scene_id)));  // its pointers are captured
         key.push_back((1ull << 60) | (uint64_t(set) << 8) | uint64_t(part));
         ve_ctx::GraphEntry* ge = nullptr;
@@ -3684,10 +3723,28 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         VE_CUDA(cudaGraphLaunch(ge->exec, st));
         return VE_OK;
     };
-    if (!pipe) {
+    if (!pipe && !early) {
         if ((rc = run(0))) return rc;
     } else {
         if ((rc = run(1))) return rc;
+        if (early) {
+            VE_CUDA(cudaEventRecord(c->frame_done, st));
+            VE_CUDA(cudaStreamWaitEvent(c->copy_stream, c->frame_done, 0));
+            uint64_t pb = 0;
+            for (uint32_t i = 0; i < nv; i++) {
+                const uint64_t np = uint64_t(views[i].frame.width) * views[i].frame.height;
+                if (outs[i].voxel_id)
+                    VE_CUDA(cudaMemcpyAsync(outs[i].voxel_id, a.out_vid + pb, np * 4, cudaMemcpyDeviceToHost, c->copy_stream));
+                if (outs[i].hit_node)
+                    VE_CUDA(cudaMemcpyAsync(outs[i].hit_node, a.out_node + pb, np * 4, cudaMemcpyDeviceToHost, c->copy_stream));
+                pb += np;
+            }
+            d2h += early_bytes;
+        }
+    }
+    if (!pipe) {
+        if (early && (rc = run(2))) return rc;
+    } else {
         // the other set's frame: its deposits and AvgPass before this decay
         VE_CUDA(cudaStreamWaitEvent(st, c->set_cache_done[set ^ 1], 0));
         if ((rc = run(2))) return rc;
@@ -3748,8 +3805,8 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
                 continue;
             }
             if (o.gbuffer) { VE_CUDA(cudaMemcpyAsync(o.gbuffer, c->gbuf.p + pb, np * 16, cudaMemcpyDeviceToHost, st)); d2h += np * 16; }
-            if (o.voxel_id) { VE_CUDA(cudaMemcpyAsync(o.voxel_id, c->out_vid.p + pb, np * 4, cudaMemcpyDeviceToHost, st)); d2h += np * 4; }
-            if (o.hit_node) { VE_CUDA(cudaMemcpyAsync(o.hit_node, c->out_node.p + pb, np * 4, cudaMemcpyDeviceToHost, st)); d2h += np * 4; }
+            if (o.voxel_id && !early) { VE_CUDA(cudaMemcpyAsync(o.voxel_id, c->out_vid.p + pb, np * 4, cudaMemcpyDeviceToHost, st)); d2h += np * 4; }
+            if (o.hit_node && !early) { VE_CUDA(cudaMemcpyAsync(o.hit_node, c->out_node.p + pb, np * 4, cudaMemcpyDeviceToHost, st)); d2h += np * 4; }
             if (o.rgb) { VE_CUDA(cudaMemcpyAsync(o.rgb, c->out_rgb.p + 3 * pb, np * 12, cudaMemcpyDeviceToHost, st)); d2h += np * 12; }
             if (o.mapped) { VE_CUDA(cudaMemcpyAsync(o.mapped, c->out_mapped.p + 3 * pb, np * 12, cudaMemcpyDeviceToHost, st)); d2h += np * 12; }
             if (o.mapped8) { VE_CUDA(cudaMemcpyAsync(o.mapped8, c->out_m8.p + pb, np * 4, cudaMemcpyDeviceToHost, st)); d2h += np * 4; }
@@ -3761,6 +3818,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
             qb += nq;
         }
         VE_CUDA(cudaStreamSynchronize(st));
+        if (early) VE_CUDA(cudaStreamSynchronize(c->copy_stream));
     }
     if (set == 1) {
         VE_CUDA(cudaEventRecord(c->alt_done, st));
