@@ -90,8 +90,9 @@ __device__ __forceinline__ float luminance(float r, float g, float b) {
 }
 
 // rUpdate / rCombine / rCapHistory (shade.comp:316-370)
+template <class R>
 __device__ __forceinline__ void r_update(Reservoir& r, uint32_t li, uint32_t lv, uint32_t seed, float target, float w,
-                                         uint32_t& rng) {
+                                         R& rng) {
     if (w <= 0.0f) {
         r.m += 1u;
         return;
@@ -105,7 +106,8 @@ __device__ __forceinline__ void r_update(Reservoir& r, uint32_t li, uint32_t lv,
         r.target = target;
     }
 }
-__device__ __forceinline__ void r_combine(Reservoir& a, const Reservoir& b, float target_at_us, uint32_t& rng) {
+template <class R>
+__device__ __forceinline__ void r_combine(Reservoir& a, const Reservoir& b, float target_at_us, R& rng) {
     if (b.m == 0u || b.target <= 0.0f || target_at_us <= 0.0f) return;
     const float w = target_at_us * b.wsum / b.target;
     a.wsum += w;

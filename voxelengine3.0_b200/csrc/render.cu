@@ -25,6 +25,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/ve.h"
@@ -724,7 +725,7 @@ __device__ __forceinline__ void nee_pending(const FrameArgs& a, uint32_t p, f3 c
 __device__ __forceinline__ void emissive_nee(const FrameArgs& a, const DevView& v, const DevScene& S, uint32_t p,
                                              uint32_t primary_vid, uint32_t b, uint32_t hx, uint32_t hy, uint32_t hz,
                                              f3 N, f3 sp, f3 dir, f3 tp, f3 albedo, float roughness, float metallic,
-                                             float spec, uint32_t& rng, uint32_t& nf, ShadeOut& o) {
+                                             float spec, RngCall& rng, uint32_t& nf, ShadeOut& o) {
     const uint32_t n_lights = min(S.em_state[0], kEmCapacity);
     if (n_lights == 0u) return;  // frame-0 pre-discovery
     const EmLight* lights = S.em_list;
@@ -991,11 +992,14 @@ __device__ __forceinline__ void shade_step(const FrameArgs& a, uint32_t p, uint4
                     }
                 }
             }
-            uint32_t rng = meta.y;
+            using Rng = std::conditional_t<EM, RngCall, uint32_t>;
+            Rng rng{meta.y};
             if (EM && (v.flags & VE_FRAME_EMISSIVE)) {
-                if (!ended && !emissive && b < 2u)
-                    emissive_nee(a, v, S, p, meta.x, b, hit.z & 0xFFFFu, hit.z >> 16, hit.w & 0xFFFFu, N, sp, dir, tp,
-                                 albedo, roughness, metallic, spec, rng, nf, o);
+                if constexpr (EM) {
+                    if (!ended && !emissive && b < 2u)
+                        emissive_nee(a, v, S, p, meta.x, b, hit.z & 0xFFFFu, hit.z >> 16, hit.w & 0xFFFFu, N, sp, dir, tp,
+                                     albedo, roughness, metallic, spec, rng, nf, o);
+                }
             } else if (!ended && !emissive && b < 2u && dot(N, sun) > 0.0f) {
                 const f3 brdf = evaluate_brdf(dir, sun, N, albedo, roughness, metallic, spec);
                 f3 c = muls(brdf, v.sun_intensity);
@@ -1068,7 +1072,7 @@ __device__ __forceinline__ void shade_step(const FrameArgs& a, uint32_t p, uint4
                 else if (!direct_stored) a.p_direct[p] = st3(direct);
                 if (pos_zero(indirect)) nf |= F_IZERO;
                 else a.p_indirect[p] = st3(indirect);
-                meta.y = rng;
+                meta.y = rng_state(rng);
                 meta.z = vi | (b << 16) | (nf << 24);
                 a.p_meta[p] = meta;
             }
