@@ -111,7 +111,7 @@ struct DevView {
 };
 
 enum : uint32_t { kMaxPasses = 18, kMaxControlChecks = 65536 };
-constexpr uint32_t kDefaultRefill = 20;  // trace refill threshold (idle lanes of 32)
+constexpr uint32_t kDefaultRefill = 24;  // trace refill threshold (idle lanes of 32)
 enum : uint32_t {
     CNT_LIVE = 0, CNT_RAY = 20, CNT_CURSOR = 40, CNT_NRC_Q = 60, CNT_NRC_S = 61, CNT_SCHED = 62, CNT_RES = 63,
     CNT_RAYSH = 64,  // shadow rays per pass (extension rays: CNT_RAY)
@@ -3059,10 +3059,10 @@ static void apply_launch(ve_ctx* c) {
     c->grid_trace_one = c->num_sms * pick(c->launch.trace_blocks_per_sm, c->occ_trace_one);
     c->grid_trace_count = c->num_sms * pick(c->launch.trace_blocks_per_sm, c->occ_trace_count);
     c->grid_shade = c->num_sms * pick(c->launch.shade_blocks_per_sm, c->occ_shade);
-    // default: refill when 20 of 32 lanes are idle (measured on the depth-10
-    // 1080p workload with the FLAT walk: 0.979 ms of trace per frame at 20
-    // against 0.984 at 16 and 0.994 at 12; each refill is a dependent chain
-    // of loads, and the cheaper the step, the fewer refills pay)
+    // default: refill when 24 of 32 lanes are idle (ms of trace per 1080p depth-10
+    // frame at 16 / 20 / 24 / 28: 0.527 / 0.508 / 0.495 / 0.515; 2160p 8 spp at
+    // 20 / 24: 2.76 / 2.69): a refill and the stores before it run once for all
+    // the idle lanes
     if (c->launch.refill_threshold == 0 || c->launch.refill_threshold > 32) c->launch.refill_threshold = kDefaultRefill;
 }
 
