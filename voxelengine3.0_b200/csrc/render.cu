@@ -224,6 +224,7 @@ struct FrameArgs {
     uint2* shade_list;      // {vid, pixel} per path
     uint32_t shade_cap;
     float* rank;            // the scene's {t_high, t_mid, histogram[256]} (thresholds from the previous frame)
+    bool own_rays;          // small trace passes may give each warp its rays (k_trace)
     bool early_ids;         // the primary pass writes out_vid / out_node (kEarlyIds), not the AvgPass
     FlatScene one;          // the batch's scene when all its views share one whose table reaches the leaves
 };
@@ -469,8 +470,12 @@ __global__ void __launch_bounds__(256) k_decay(CacheEntry* cache, uint32_t n, fl
 // registers and 8 CTAs/SM (0.637 -> 0.606 ms of trace per 1080p depth-10 frame;
 // at 6 CTAs/SM 0.641, so it is the resident warps that pay: the walk waits on
 // its loads).
-// A warp's first 32 rays are fixed: with 9472 warps at the cursor from the
-// start, the trace of a 256x256 depth-7 frame took 0.056 ms instead of 0.047.
+// Small passes hand each warp its first rays: with 9472 warps at the cursor, the
+// trace of a 256x256 depth-7 frame took 0.039 ms instead of 0.037, of a 512x512
+// emissive one 0.157 instead of 0.148; large passes do not care.  Not in
+// pipelined frames (own_rays): there another kernel may hold SMs, and a warp that
+// is not resident must not own rays — with fixed first rays for every pass, some
+// runs of pipelined 1080p frames took 1.87 ms a frame instead of 1.04.
 enum : uint32_t { kLaneIdle = 4u };  // lane state: kWalking, a finished ray's status to be stored, or no ray
 template <bool COUNT, bool EM = false, bool FLAT = false, bool ONE = false>
 __global__ void __launch_bounds__(256, ONE ? 8 : 6) k_trace(FrameArgs a, uint32_t pass) {
@@ -483,11 +488,11 @@ __global__ void __launch_bounds__(256, ONE ? 8 : 6) k_trace(FrameArgs a, uint32_
     uint32_t* cursor = &a.counters[CNT_CURSOR + pass];
     const uint32_t lane = lane_id();
     bool drained = false;  // warp-uniform: every ray of the pass has been handed out
-    // the first 32 rays of each warp are its own, so a pass with less than a
-    // grid of them touches no cursor; the cursor hands out the rest
-    const uint32_t own = gridDim.x * blockDim.x;
-    uint32_t first_idx = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;
-    bool first = true;
+    // a pass of at most four rays per lane: each warp's first 32 are its own, the
+    // cursor hands out the rest (`fixed` on)
+    const uint32_t lanes = gridDim.x * blockDim.x;
+    const uint32_t fixed = a.own_rays && n <= 4u * lanes ? lanes : 0u;
+    bool own = fixed != 0u;
     uint32_t state = kLaneIdle;
     uint32_t D = 0, T0 = 0;
     const uint32_t* nodes = nullptr;
@@ -532,13 +537,14 @@ __global__ void __launch_bounds__(256, ONE ? 8 : 6) k_trace(FrameArgs a, uint32_
         if (drained) break;  // the last rays have just been stored
         const unsigned idle = __ballot_sync(0xffffffffu, state == kLaneIdle);
         const uint32_t want = uint32_t(__popc(idle));
-        if (!first) {
+        uint32_t first_idx = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;
+        if (!own) {
             const int leader = __ffs(idle) - 1;
-            if (int(lane) == leader) first_idx = own + atomicAdd(cursor, want);
+            if (int(lane) == leader) first_idx = fixed + atomicAdd(cursor, want);
             first_idx = __shfl_sync(0xffffffffu, first_idx, leader);
         }
-        drained = first ? own >= n : first_idx + want >= n;
-        first = false;
+        drained = (own ? fixed : first_idx + want) >= n;
+        own = false;
         if (state == kLaneIdle) {
             const uint32_t idx = first_idx + uint32_t(__popc(idle & ((1u << lane) - 1u)));
             if (idx < n) {
@@ -3589,6 +3595,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         a.res_list = c->res_list.p;
     }
     a.early_ids = early;
+    a.own_rays = !pipe;
     one = one && flat;
     if (one) {
         const SceneSlot& sc = c->scenes[views[0].scene_id];
@@ -3739,7 +3746,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         key.push_back((1ull << 61) | uint64_t(parity));
         key.push_back((1ull << 59) | (uint64_t(early) << 1) | uint64_t(flat));
         if (one) key.push_back((1ull << 58) | uint64_t(uint32_t(views[0].scene_id)));  // its pointers are captured
-        key.push_back((1ull << 60) | (uint64_t(set) << 8) | uint64_t(part));
+        key.push_back((1ull << 60) | (uint64_t(pipe) << 16) | (uint64_t(set) << 8) | uint64_t(part));
         ve_ctx::GraphEntry* ge = nullptr;
         for (auto& g : c->graphs)
             if (g.key == key) ge = &g;
