@@ -261,11 +261,10 @@ __device__ __forceinline__ void warp_add_stat(unsigned long long* stat, uint32_t
 __device__ __forceinline__ uint32_t cache_home(uint32_t vid, uint32_t log2n) {
     return (vid * 0x9E3779B1u) >> (32u - log2n);
 }
-__device__ __forceinline__ int cache_claim(CacheEntry* c, uint32_t log2n, uint32_t probes, uint32_t vid) {
+// `fresh`: this call claimed the slot, which cache_list then adds to the list.
+__device__ __forceinline__ int cache_claim(CacheEntry* c, uint32_t log2n, uint32_t probes, uint32_t vid, bool& fresh) {
     const uint32_t mask = (1u << log2n) - 1u;
     const uint32_t h = cache_home(vid, log2n);
-    int slot = -1;
-    bool fresh = false;
     for (uint32_t i = 0; i < probes; i++) {
         const uint32_t s = (h + i) & mask;
         uint32_t k = *((volatile uint32_t*)&c[s].key);
@@ -273,23 +272,24 @@ __device__ __forceinline__ int cache_claim(CacheEntry* c, uint32_t log2n, uint32
             k = atomicCAS(&c[s].key, 0u, vid);
             fresh = k == 0u;
         }
-        if (fresh || k == vid) {
-            slot = int(s);
-            break;
-        }
+        if (fresh || k == vid) return int(s);
     }
-    if (fresh) {
-        // the claimed slot joins the list; the lanes here at once that claim
-        // from the same table share an atomic
-        const unsigned here = __activemask();
-        const unsigned peers = __match_any_sync(here, reinterpret_cast<unsigned long long>(c));
-        const int first = __ffs(peers) - 1;
-        uint32_t at = 0;
-        if (int(lane_id()) == first) at = atomicAdd(&c[mask + 1u].count, uint32_t(__popc(peers)));
-        at = __shfl_sync(peers, at, first) + uint32_t(__popc(peers & ((1u << lane_id()) - 1u)));
-        if (at <= mask) c[at].used = uint32_t(slot);
-    }
-    return slot;
+    return -1;
+}
+// The slots a warp's lanes have just claimed join their tables' lists, one
+// atomic per table.  Called by all 32 lanes of a warp: the lanes leave the
+// claims' probe loops at different times, and none of them may be counted on
+// to be there with another before they meet again.
+__device__ __forceinline__ void cache_list(bool fresh, CacheEntry* c, uint32_t log2n, int slot) {
+    const unsigned all = __ballot_sync(0xffffffffu, fresh);
+    if (all == 0u) return;
+    const unsigned peers = all & __match_any_sync(0xffffffffu, fresh ? reinterpret_cast<unsigned long long>(c) : 0ull);
+    const int first = __ffs(peers) - 1;  // -1: a lane without a claim
+    const uint32_t mask = (1u << log2n) - 1u;
+    uint32_t at = 0;
+    if (int(lane_id()) == first) at = atomicAdd(&c[mask + 1u].count, uint32_t(__popc(peers)));
+    at = __shfl_sync(0xffffffffu, at, first & 31) + uint32_t(__popc(peers & ((1u << lane_id()) - 1u)));
+    if (fresh && at <= mask) c[at].used = uint32_t(slot);
 }
 __device__ __forceinline__ int cache_find(const CacheEntry* c, uint32_t log2n, uint32_t probes, uint32_t vid) {
     const uint32_t mask = (1u << log2n) - 1u;
@@ -340,12 +340,18 @@ __device__ __forceinline__ void warp_deposit(bool active, uint32_t scene, uint32
     const bool last = lane == 31 || ((heads >> (lane + 1)) & 1u);
     vid = __shfl_sync(0xffffffffu, vid, start & 31);
     scene = __shfl_sync(0xffffffffu, scene, start & 31);
+    bool fresh = false;
+    int s = -1;
+    CacheEntry* cache = nullptr;
+    uint32_t log2n = 0;
     if (last && start >= 0) {
         const uint32_t n = uint32_t(__popc(am & (lt | (1u << lane)) & ~((1u << start) - 1u)));
         const DevScene& S = scenes[scene];
-        const int s = cache_claim(S.cache, S.cache_log2, S.probes, vid);
+        cache = S.cache;
+        log2n = S.cache_log2;
+        s = cache_claim(cache, log2n, S.probes, vid, fresh);
         if (s >= 0) {
-            CacheEntry* e = S.cache + s;
+            CacheEntry* e = cache + s;
             atomicAdd(&e->count, n);
             atomicAdd(&e->l2, l2);
             atomicAdd(&e->rgbw, make_float4(r, g, b, float(n)));
@@ -354,6 +360,7 @@ __device__ __forceinline__ void warp_deposit(bool active, uint32_t scene, uint32
             n_drop += n;
         }
     }
+    cache_list(fresh, cache, log2n, s);
 }
 
 // Per-thread tallies of a shading kernel, added to the frame's counters once
@@ -3944,19 +3951,27 @@ __global__ void __launch_bounds__(256) k_split_export(CacheEntry* __restrict__ t
 __global__ void __launch_bounds__(256) k_split_merge(CacheEntry* cache, uint32_t log2n, uint32_t probes,
                                                      const uint4* __restrict__ rec, uint32_t n, uint32_t* dropped) {
     uint32_t drops = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint4 a = rec[2ull * i + 0], b = rec[2ull * i + 1];
-        if (a.x == 0u || a.y == 0u) continue;
-        const int s = cache_claim(cache, log2n, probes, a.x);
-        if (s < 0) {
-            drops++;
-            continue;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {  // uniform per warp
+        uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
+        if (threadIdx.x < n - base) {
+            a = rec[2ull * (base + threadIdx.x) + 0];
+            b = rec[2ull * (base + threadIdx.x) + 1];
         }
-        CacheEntry* e = cache + s;
-        atomicAdd(&e->count, a.y);
-        atomicAdd(&e->l2, __uint_as_float(a.z));
-        atomicAdd(&e->rgbw, make_float4(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y),
-                                        __uint_as_float(b.z)));
+        bool fresh = false;
+        int s = -1;
+        if (a.x != 0u && a.y != 0u) {
+            s = cache_claim(cache, log2n, probes, a.x, fresh);
+            if (s >= 0) {
+                CacheEntry* e = cache + s;
+                atomicAdd(&e->count, a.y);
+                atomicAdd(&e->l2, __uint_as_float(a.z));
+                atomicAdd(&e->rgbw, make_float4(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y),
+                                                __uint_as_float(b.z)));
+            } else {
+                drops++;
+            }
+        }
+        cache_list(fresh, cache, log2n, s);
     }
     if (drops) atomicAdd(dropped, drops);
 }
