@@ -3794,6 +3794,10 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
     if (!pipe && !early) {
         if ((rc = run(0))) return rc;
     } else {
+        // the frame sets share the id images: part 1 writes them early only once
+        // the other set's frame, which may still be on its way (one without
+        // outputs is not waited for), has written its own
+        if (early && pipe) VE_CUDA(cudaStreamWaitEvent(st, c->set_cache_done[set ^ 1], 0));
         if ((rc = run(1))) return rc;
         if (early) {
             VE_CUDA(cudaEventRecord(c->frame_done, st));
