@@ -611,12 +611,15 @@ def _dev_ptr(buf) -> Optional[int]:
     return int(buf)
 
 
-def _alloc_outputs(fc: FrameConfig, want: Iterable[str]):
+def _alloc_outputs(fc: FrameConfig, want: Iterable[str], call_flags: int):
+    """Host arrays for one view's outputs; `call_flags`: the flags of all the
+    call's views together."""
     npx = fc.width * fc.height
     arrays: Dict[str, np.ndarray] = {}
     # a split frame writes its band's rows only; asynchronous copies land after
-    # the call, when nothing here would keep their array
-    new = np.zeros if fc.flags & (FRAME_SPLIT | FRAME_ASYNC_OUTPUTS) else _results.empty
+    # the call, when nothing here would keep their array, and a call is
+    # asynchronous for all its views when one of them asks for it
+    new = np.zeros if call_flags & (FRAME_SPLIT | FRAME_ASYNC_OUTPUTS) else _results.empty
     for k in want:
         if k == "gbuffer":
             arrays[k] = new((fc.height, fc.width, 4), np.uint32)
@@ -819,7 +822,7 @@ class Renderer:
         """One frame of one view; returns the requested host outputs."""
         view = self.make_view(scene_id, camera, fc)
         want = list(outputs)
-        o, arrays = _alloc_outputs(fc, want)
+        o, arrays = _alloc_outputs(fc, want, fc.flags)
         self._check_copied(self._lib.ve_render(self._h, ctypes.byref(view), ctypes.byref(o) if want else None))
         return arrays
 
@@ -838,9 +841,12 @@ class Renderer:
         want = list(outputs)
         outs = (FrameOutputsC * len(views))()
         results: List[Dict[str, np.ndarray]] = []
+        call_flags = 0
+        for _, _, fc in views:
+            call_flags |= fc.flags
         for i, (sid, cam, fc) in enumerate(views):
             arr[i] = self.make_view(sid, cam, fc)
-            o, arrays = _alloc_outputs(fc, want)
+            o, arrays = _alloc_outputs(fc, want, call_flags)
             outs[i] = o
             results.append(arrays)
         self._check_copied(self._lib.ve_render_batch(self._h, arr, len(views), outs if want else None))
@@ -870,7 +876,7 @@ class Renderer:
         images with the band's rows written."""
         view = self.make_view(scene_id, camera, fc)
         want = list(outputs)
-        o, arrays = _alloc_outputs(fc, want)
+        o, arrays = _alloc_outputs(fc, want, fc.flags)
         _check(self._lib.ve_split_resolve(self._h, ctypes.byref(view), ctypes.byref(o) if want else None))
         return arrays
 
