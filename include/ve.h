@@ -256,7 +256,8 @@ int ve_ctx_synchronize(ve_ctx* ctx);
 /* Orders work enqueued on the context's stream after this call behind every
  * frame rendered so far (VE_CFG_PIPELINE runs some on a second stream). */
 int ve_ctx_join(ve_ctx* ctx);
-/* Pinned host memory for result arrays (any context may copy into it; freed
+/* Pinned host memory for result arrays (any context may copy into it; a forked
+ * child has its own copy; freed
  * by the caller once no copy into it is in flight). */
 int ve_host_alloc(uint64_t bytes, void** out);
 int ve_host_free(void* p);
