@@ -17,6 +17,7 @@ libve.so, and loading fails loudly when the library is missing.
 """
 from __future__ import annotations
 
+import collections
 import ctypes
 import dataclasses
 import math
@@ -286,8 +287,13 @@ class _ResultPool:
     on every call.  A pinned one is written by the GPU directly, and is used
     again once the program has dropped the arrays it was under: a call with 12
     mixed views (165 MB of results) takes 5.4 ms instead of 25, 1 M rays 2.6
-    instead of 6.5, a 256x256 frame 0.17 instead of 0.41.  At most LIMIT bytes are
-    held, in use or not; beyond that, and under MIN bytes (where a pageable copy
+    instead of 6.5, a 256x256 frame 0.17 instead of 0.41.
+
+    Pinning a new block costs what three to five calls then save, so a size is
+    pinned when it is asked for the second time, and its first call costs what
+    it does with ordinary arrays.  A free block serves any size from half its
+    own up.  At most LIMIT bytes are held, in use or not, the free blocks longest
+    unused making room; beyond that, and under MIN bytes (where a pageable copy
     is as quick), results come in ordinary arrays.  The blocks not in use are
     freed when the last Renderer is closed.
     """
@@ -296,9 +302,14 @@ class _ResultPool:
     LIMIT = 512 << 20
 
     def __init__(self):
-        self._lock = threading.RLock()  # re-entered when a collection inside ends a block
-        self._free: Dict[int, List[int]] = {}
+        self._lock = threading.Lock()
+        # blocks given back: a collection may end one anywhere, inside these
+        # methods too, so the owner only leaves it here for whoever has the lock
+        self._returned: collections.deque = collections.deque()
+        self._free: Dict[int, List[tuple]] = {}  # size -> (time given back, address), oldest first
+        self._asked: set = set()  # sizes asked for before
         self._held = 0
+        self._time = 0
         self._renderers = 0
 
     @staticmethod
@@ -310,39 +321,74 @@ class _ResultPool:
         """An array for results that the library writes whole."""
         dtype = np.dtype(dtype)
         n = dtype.itemsize * math.prod(shape)
-        block = self._take(self._size_class(n)) if n >= self.MIN else None
+        block = None
+        if n >= self.MIN:
+            with self._lock:
+                block = self._take(self._size_class(n))
+            self._settle()
         if block is None:
             return np.zeros(shape, dtype)
         return np.asarray(block)[:n].view(dtype).reshape(shape)
 
     def _take(self, size: int) -> Optional[_PinnedBlock]:
-        with self._lock:
-            free = self._free.get(size)
-            if free:
-                return _PinnedBlock(self, free.pop(), size)
-            if self._held + size > self.LIMIT:
-                self._trim()
-            if self._held + size > self.LIMIT:
-                return None
-            p = _P()
-            if load_library().ve_host_alloc(size, ctypes.byref(p)) != VE_OK:
-                return None
-            self._held += size
-            return _PinnedBlock(self, p.value, size)
+        self._collect()
+        s = size
+        while s <= 2 * size:
+            if s in self._free:
+                return _PinnedBlock(self, self._pop(s, -1), s)
+            s = self._size_class(s + 1)
+        if size not in self._asked:
+            self._asked.add(size)
+            return None
+        if size > self.LIMIT:
+            return None
+        while self._free and self._held + size > self.LIMIT:
+            self._release(min(self._free, key=lambda k: self._free[k][0]))
+        if self._held + size > self.LIMIT:
+            return None
+        p = _P()
+        if load_library().ve_host_alloc(size, ctypes.byref(p)) != VE_OK:
+            return None
+        self._held += size
+        return _PinnedBlock(self, p.value, size)
+
+    def _pop(self, size: int, at: int) -> int:
+        blocks = self._free[size]
+        ptr = blocks.pop(at)[1]
+        if not blocks:
+            del self._free[size]
+        return ptr
 
     def give(self, ptr: int, size: int) -> None:
-        with self._lock:
-            self._free.setdefault(size, []).append(ptr)
-            if self._renderers == 0:
-                self._trim()
+        self._returned.append((ptr, size))
+        self._settle()
+
+    def _settle(self) -> None:
+        """Files the blocks given back, unless who has the lock will do it."""
+        while self._returned and self._lock.acquire(blocking=False):
+            try:
+                self._collect()
+            finally:
+                self._lock.release()
+
+    def _collect(self) -> None:
+        while self._returned:
+            ptr, size = self._returned.popleft()
+            self._time += 1
+            self._free.setdefault(size, []).append((self._time, ptr))
+        if self._renderers == 0:
+            self._trim()
+
+    def _release(self, size: int) -> None:
+        """Frees the free block of this size that is longest unused."""
+        ptr = self._pop(size, 0)
+        if _lib is not None:
+            _lib.ve_host_free(ptr)
+        self._held -= size
 
     def _trim(self) -> None:
-        free, self._free = self._free, {}
-        for size, ptrs in free.items():
-            for p in ptrs:
-                if _lib is not None:
-                    _lib.ve_host_free(p)
-                self._held -= size
+        while self._free:
+            self._release(next(iter(self._free)))
 
     def opened(self) -> None:
         with self._lock:
@@ -352,7 +398,9 @@ class _ResultPool:
         with self._lock:
             self._renderers -= 1
             if self._renderers == 0:
-                self._trim()
+                self._asked.clear()
+            self._collect()
+        self._settle()
 
 
 _results = _ResultPool()
