@@ -56,3 +56,33 @@ def test_a_forked_child_keeps_its_copy(ve, size):
         del image
         assert ve.load_library().ve_host_free(p) == ve.VE_OK
         assert ve.load_library().ve_host_free(p) != ve.VE_OK  # no longer a block
+
+
+@pytest.mark.gpu
+def test_blocks_made_and_freed_by_a_fresh_thread(ve):
+    """A thread that has made no CUDA call takes a renderer's device."""
+    import threading
+
+    words, depth, mats, cam, fc = helpers.small_setup()
+    fc.width, fc.height = 300, 200
+    rc = []
+
+    def work():
+        p = ctypes.c_void_p()
+        rc.append(ve.load_library().ve_host_alloc(300 * 200 * 4, ctypes.byref(p)))
+        image = np.frombuffer((ctypes.c_char * (300 * 200 * 4)).from_address(p.value), np.uint32).reshape(200, 300)
+        r.render_into(sid, cam, fc, {"voxel_id": image})
+        rc.append(np.array_equal(image, want))
+        del image
+        t = threading.Thread(target=lambda: rc.append(ve.load_library().ve_host_free(p)))
+        t.start()
+        t.join(60)
+
+    with ve.Renderer(hash_log2=16) as r:
+        r.set_materials(mats)
+        sid = r.upload_scene(words, depth)
+        want = r.render(sid, cam, fc, outputs=("voxel_id",))["voxel_id"].copy()
+        t = threading.Thread(target=work)
+        t.start()
+        t.join(60)
+    assert rc == [ve.VE_OK, True, ve.VE_OK]

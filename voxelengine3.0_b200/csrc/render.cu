@@ -23,6 +23,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <type_traits>
@@ -2349,6 +2350,7 @@ constexpr size_t kScratchLarge = 128u << 20;  // larger pieces are allocated and
 
 struct ve_ctx {
     int device = 0;
+    bool counted = false;  // among the live contexts (count_live)
     cudaMemPool_t scratch = nullptr;  // stream-ordered scratch of scene builds and normal passes
     int num_sms = 148;
     cudaStream_t stream = nullptr;
@@ -3995,6 +3997,8 @@ extern "C" {
 
 const char* ve_last_error(void) { return g_err.c_str(); }
 
+static void count_live(int device, int by);
+
 int ve_ctx_create(const ve_renderer_config* cfg, ve_ctx** out) {
     if (!out) return fail(VE_ERR_INVALID, "ctx_create: null output");
     *out = nullptr;
@@ -4106,12 +4110,15 @@ int ve_ctx_create(const ve_renderer_config* cfg, ve_ctx** out) {
         ve_ctx_destroy(x);
         return fail(VE_ERR_CUDA, "ctx_create: initialisation failed");
     }
+    count_live(x->device, 1);
+    x->counted = true;
     *out = x;
     return VE_OK;
 }
 
 int ve_ctx_destroy(ve_ctx* c) {
     if (!c) return VE_OK;
+    if (c->counted) count_live(c->device, -1);
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     while (!c->nrcs.empty()) ve_nrc_destroy(c->nrcs.back());
@@ -4190,6 +4197,23 @@ int ve_ctx_join(ve_ctx* c) {
     return VE_OK;
 }
 
+using CtxGetCurrentFn = CUresult (*)(CUcontext*);
+
+// the calling thread's current driver context (null when none is current)
+static void* current_ctx() {
+    static CtxGetCurrentFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<CtxGetCurrentFn>(f);
+    }();
+    CUcontext c = nullptr;
+    if (!fn || fn(&c) != CUDA_SUCCESS) return nullptr;
+    return c;
+}
+
 // Private pages made by the kernel and then pinned, from 2 MB on in huge pages:
 // cudaHostAlloc takes about 0.7 ms a MB (32 MB: 20..34 ms), which the first
 // call of each result size would pay; this way it is 5.2 ms, 4.0 of them the
@@ -4198,6 +4222,25 @@ int ve_ctx_join(ve_ctx* c) {
 static std::mutex g_host_mu;
 static std::unordered_map<void*, std::pair<void*, size_t>> g_host;  // block -> its mapping
 constexpr size_t kHugePage = 2u << 20;
+static std::map<int, int> g_live;  // device -> live renderer contexts on it (under g_host_mu)
+
+static void count_live(int device, int by) {
+    std::lock_guard<std::mutex> lock(g_host_mu);
+    if ((g_live[device] += by) == 0) g_live.erase(device);
+}
+
+// Pinning needs a device, any of them.  A thread that has none yet (a program's
+// render thread, before its first call) takes one that has a renderer: the
+// runtime's default would make a context on device 0, in every rank.
+static void bind_live_device() {
+    if (current_ctx()) return;
+    int device = -1;
+    {
+        std::lock_guard<std::mutex> lock(g_host_mu);
+        if (!g_live.empty()) device = g_live.begin()->first;
+    }
+    if (device >= 0) cudaSetDevice(device);
+}
 
 int ve_host_alloc(uint64_t bytes, void** out) {
     if (!out || bytes == 0) return fail(VE_ERR_INVALID, "host_alloc: null output or no bytes");
@@ -4209,6 +4252,7 @@ int ve_host_alloc(uint64_t bytes, void** out) {
     if (base == MAP_FAILED) return fail(VE_ERR_NOMEM, "host_alloc: pinned allocation failed");
     void* p = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(base) + align - 1) & ~uintptr_t(align - 1));
     if (align == kHugePage) madvise(p, size, MADV_HUGEPAGE);
+    bind_live_device();
     if (cudaHostRegister(p, size, cudaHostRegisterPortable) != cudaSuccess) {
         cudaGetLastError();
         munmap(base, len);
@@ -4230,6 +4274,7 @@ int ve_host_free(void* p) {
         map = it->second;
         g_host.erase(it);
     }
+    bind_live_device();
     if (cudaHostUnregister(p) != cudaSuccess) cudaGetLastError();  // (the context is gone, and its pins with it)
     munmap(map.first, map.second);
     return VE_OK;
@@ -5093,22 +5138,6 @@ struct NoAllocSlot {
 };
 static NoAllocSlot g_noalloc_slot[64] = {};
 static std::mutex g_noalloc_mu;
-using CtxGetCurrentFn = CUresult (*)(CUcontext*);
-
-// the calling thread's current driver context (null when none is current)
-static void* noalloc_current_ctx() {
-    static CtxGetCurrentFn fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            f = nullptr;
-        return reinterpret_cast<CtxGetCurrentFn>(f);
-    }();
-    CUcontext c = nullptr;
-    if (!fn || fn(&c) != CUDA_SUCCESS) return nullptr;
-    return c;
-}
 
 int ve_fill_normals_noalloc(uint32_t* words, uint64_t n_words, uint32_t depth, void* stream) {
     if (!words) return fail(VE_ERR_INVALID, "fill_normals_noalloc: null node array");
@@ -5124,7 +5153,7 @@ int ve_fill_normals_noalloc(uint32_t* words, uint64_t n_words, uint32_t depth, v
     {
         std::lock_guard<std::mutex> lock(g_noalloc_mu);
         NoAllocSlot& slot = g_noalloc_slot[dev];
-        void* ctx = noalloc_current_ctx();
+        void* ctx = current_ctx();
         if (!slot.ptr || !ctx || ctx != slot.ctx) {
             void* p = nullptr;
             cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
@@ -5132,7 +5161,7 @@ int ve_fill_normals_noalloc(uint32_t* words, uint64_t n_words, uint32_t depth, v
                 return fail(VE_ERR_CUDA, std::string("fill_normals_noalloc: cudaGetSymbolAddress: ") +
                                              cudaGetErrorString(e));
             // the lookup makes the device's primary context current when none was
-            slot.ctx = ctx ? ctx : noalloc_current_ctx();
+            slot.ctx = ctx ? ctx : current_ctx();
             slot.ptr = p;
         }
         base = slot.ptr;
