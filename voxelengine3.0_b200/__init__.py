@@ -943,7 +943,8 @@ class Renderer:
 
     def set_launch_config(self, trace_blocks_per_sm: int = 0, shade_blocks_per_sm: int = 0,
                           refill_threshold: int = 0) -> None:
-        """0 for any field keeps the library's default (occupancy maximum; refill at 24 idle lanes)."""
+        """0 for any field keeps the library's default (occupancy maximum; refill at 24 idle lanes, 20 where a
+        scene's top table does not reach its leaves)."""
         c = LaunchConfigC(trace_blocks_per_sm, shade_blocks_per_sm, refill_threshold, 0)
         _check(self._lib.ve_set_launch_config(self._h, ctypes.byref(c)))
 

@@ -116,7 +116,16 @@ struct DevView {
 };
 
 enum : uint32_t { kMaxPasses = 18, kMaxControlChecks = 65536 };
-constexpr uint32_t kDefaultRefill = 24;  // trace refill threshold (idle lanes of 32)
+// Trace refill thresholds (idle lanes of 32).  A refill, a dependent chain of
+// loads, and the stores before it run once for all the idle lanes; the cheaper
+// the step, the more lanes may idle before that pays.  ms of trace at 12 / 16 /
+// 20 / 24 / 28: flat walk, 1080p depth 10 0.566 / 0.525 / 0.509 / 0.493 / 0.520,
+// 12 views over three scenes 1.177 / 1.058 / 1.003 / 0.978 / 1.004, emissive
+// Cornell 0.211 / 0.202 / 0.203 / 0.203 / 0.207; general walk, 1080p depth 11
+// 0.321 / 0.314 / 0.316 / 0.322 / 0.323, 12 views with depth 11 among them
+// 1.555 / 1.520 / 1.508 / 1.525 / 1.631.
+constexpr uint32_t kDefaultRefill = 24;         // flat walk
+constexpr uint32_t kDefaultRefillGeneral = 20;  // walk of every level below the table
 enum : uint32_t {
     CNT_LIVE = 0, CNT_RAY = 20, CNT_CURSOR = 40, CNT_NRC_Q = 60, CNT_NRC_S = 61, CNT_SCHED = 62, CNT_RES = 63,
     CNT_RAYSH = 64,  // shadow rays per pass (extension rays: CNT_RAY)
@@ -2439,7 +2448,7 @@ struct ve_ctx {
     int occ_trace = 1, occ_trace_one = 1, occ_trace_count = 1, occ_shade = 1;  // occupancy maxima (blocks/SM)
     int occ_shade_mode[8] = {1, 1, 1, 1, 1, 1, 1, 1};       // ... per shading instance (kModeEm | kModeLb | kModeNrc)
     int occ_emit_mode[4] = {1, 1, 1, 1};                    // ... per scheduled-emit instance
-    ve_launch_config launch{0, 0, ve::kDefaultRefill, 0};
+    ve_launch_config launch{0, 0, 0, 0};  // 0: the defaults
     // per-frame CUDA-event sets in a ring: elapsed times are read when the
     // slot is reused or the stats are queried, so timed frames never wait
     static constexpr int kTimingSlots = 16, kEvents = 48;
@@ -3128,11 +3137,12 @@ static void apply_launch(ve_ctx* c) {
     c->grid_trace_one = c->num_sms * pick(c->launch.trace_blocks_per_sm, c->occ_trace_one);
     c->grid_trace_count = c->num_sms * pick(c->launch.trace_blocks_per_sm, c->occ_trace_count);
     c->grid_shade = c->num_sms * pick(c->launch.shade_blocks_per_sm, c->occ_shade);
-    // default: refill when 24 of 32 lanes are idle (ms of trace per 1080p depth-10
-    // frame at 16 / 20 / 24 / 28: 0.527 / 0.508 / 0.495 / 0.515; 2160p 8 spp at
-    // 20 / 24: 2.76 / 2.69): a refill and the stores before it run once for all
-    // the idle lanes
-    if (c->launch.refill_threshold == 0 || c->launch.refill_threshold > 32) c->launch.refill_threshold = kDefaultRefill;
+}
+
+// Refill threshold of a trace pass: the configured one, else its walk's default.
+static uint32_t refill_of(const ve_ctx* c, bool flat) {
+    if (c->launch.refill_threshold) return c->launch.refill_threshold;
+    return flat ? kDefaultRefill : kDefaultRefillGeneral;
 }
 
 // Grid of a shading instance: the configured blocks per SM, capped at what
@@ -3564,7 +3574,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
     a.out_mapped = parity ? c->out_mapped2.p : c->out_mapped.p;
     a.out_mapped8 = parity ? c->out_m82.p : c->out_m8.p;
     a.path_rgb = (flags & VE_FRAME_PATH_RGB) ? c->path_rgb.p : nullptr;
-    a.refill = c->launch.refill_threshold;
+    a.refill = refill_of(c, flat && !count);
     a.view_offset = 0;
     a.remaining = nullptr;
     const bool learned = nrc && (flags & VE_FRAME_LEARNED);
@@ -4985,6 +4995,7 @@ int ve_split_resolve(ve_ctx* c, const ve_view* view, ve_frame_outputs* out) {
 int ve_get_launch_config(ve_ctx* c, ve_launch_config* cfg) {
     if (!c || !cfg) return fail(VE_ERR_INVALID, "get_launch_config: null argument");
     *cfg = c->launch;
+    if (cfg->refill_threshold == 0) cfg->refill_threshold = kDefaultRefill;
     return VE_OK;
 }
 

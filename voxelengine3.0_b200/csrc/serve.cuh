@@ -175,7 +175,6 @@ static FrameArgs serve_args(ve_server* s) {
     a.gbuf = c->gbuf.p; a.out_vid = c->out_vid.p; a.out_node = c->out_node.p;
     a.out_rgb = c->out_rgb.p; a.out_mapped = c->out_mapped.p;
     a.path_rgb = nullptr;
-    a.refill = c->launch.refill_threshold;
     a.view_offset = 0;
     a.remaining = s->d_remaining;
     return a;
@@ -317,6 +316,7 @@ static void serve_loop(ve_server* s) {
             const SceneSlot& sc = c->scenes[r->view.scene_id];
             flat = flat && sc.top_level != 0u && sc.top_level == sc.depth;
         }
+        a.refill = refill_of(c, flat);
         launch_trace(c, st, a, ps, false, false, flat, false);
         if (ps == kRing - 1)  // wrap: the survivors' count moves to slot 0
             cudaMemcpyAsync(c->counters.p + CNT_LIVE, c->counters.p + CNT_LIVE + kRing, 4, cudaMemcpyDeviceToDevice,
