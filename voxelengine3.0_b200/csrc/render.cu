@@ -167,6 +167,8 @@ __device__ __forceinline__ bool pos_zero(f3 v) {
 // _TERMINATE_HASH / _TRAIN); only the shade pass needs that instance, since
 // the primary and scheduled-emit passes shade vertex 0 only.
 constexpr int kModeEm = 1, kModeLb = 2, kModeNrc = 4;
+// k_trace's instances: fetch counting, one scene, scenes with a table to the leaves, any
+enum TraceKind : int { kTraceGeneral, kTraceFlat, kTraceOne, kTraceCount, kTraceKinds };
 constexpr int kShadeRowsMode = 7;  // (no batch's mode) k_shade_rows' place among the shading grids
 // a cached voxel average ends a path (VE_FRAME_TERMINATE_HASH, and the
 // learned cache's fallback) only when at least this many deposits made it
@@ -2444,8 +2446,8 @@ struct ve_ctx {
     ve::DevBuf<uint32_t> box;      // build_top: the box, the face search's result
     ve::DevBuf<float> ray_in;      // ve_raycast_batch: origins and directions
     ve::DevBuf<uint32_t> ray_out;  // ve_raycast_batch: 8 words per ray
-    int grid_trace = 0, grid_trace_one = 0, grid_trace_count = 0, grid_shade = 0;
-    int occ_trace = 1, occ_trace_one = 1, occ_trace_count = 1, occ_shade = 1;  // occupancy maxima (blocks/SM)
+    // occupancy maxima (blocks/SM): per trace instance (plain, emissive), ...
+    int occ_trace[2][ve::kTraceKinds] = {{1, 1, 1, 1}, {1, 1, 1, 1}};
     int occ_shade_mode[8] = {1, 1, 1, 1, 1, 1, 1, 1};       // ... per shading instance (kModeEm | kModeLb | kModeNrc)
     int occ_emit_mode[4] = {1, 1, 1, 1};                    // ... per scheduled-emit instance
     ve_launch_config launch{0, 0, 0, 0};  // 0: the defaults
@@ -3129,33 +3131,26 @@ static void collect_all_timing(ve_ctx* c) {
     }
 }
 
-// Grid sizes of the persistent kernels from the launch config (0 = the
-// occupancy maximum), clamped to what can be resident.
-static void apply_launch(ve_ctx* c) {
-    auto pick = [&](uint32_t want, int occ) { return int((want == 0 || int(want) > occ) ? occ : int(want)); };
-    c->grid_trace = c->num_sms * pick(c->launch.trace_blocks_per_sm, c->occ_trace);
-    c->grid_trace_one = c->num_sms * pick(c->launch.trace_blocks_per_sm, c->occ_trace_one);
-    c->grid_trace_count = c->num_sms * pick(c->launch.trace_blocks_per_sm, c->occ_trace_count);
-    c->grid_shade = c->num_sms * pick(c->launch.shade_blocks_per_sm, c->occ_shade);
+// Blocks of a persistent kernel: the configured number per SM (0: the
+// occupancy maximum), at most what its instance keeps resident, so that the
+// grid is one wave.
+static uint32_t resident_grid(const ve_ctx* c, uint32_t want, int occ) {
+    return uint32_t(c->num_sms) * ((want == 0u || want > uint32_t(occ)) ? uint32_t(occ) : want);
 }
 
 // Refill threshold of a trace pass: the configured one, else its walk's default.
-static uint32_t refill_of(const ve_ctx* c, bool flat) {
+static uint32_t refill_of(const ve_ctx* c, TraceKind kind) {
     if (c->launch.refill_threshold) return c->launch.refill_threshold;
-    return flat ? kDefaultRefill : kDefaultRefillGeneral;
+    return kind == kTraceOne || kind == kTraceFlat ? kDefaultRefill : kDefaultRefillGeneral;
 }
 
-// Grid of a shading instance: the configured blocks per SM, capped at what
-// that instance keeps resident (so the grid is one wave).
 static uint32_t shade_grid(const ve_ctx* c, int mode, bool emit) {
-    const int occ = emit ? c->occ_emit_mode[mode & 3] : c->occ_shade_mode[mode & 7];
-    const int want = int(c->launch.shade_blocks_per_sm);
-    return uint32_t(c->num_sms * ((want == 0 || want > occ) ? occ : want));
+    return resident_grid(c, c->launch.shade_blocks_per_sm, emit ? c->occ_emit_mode[mode & 3] : c->occ_shade_mode[mode & 7]);
 }
 
-static void launch_shade(const ve_ctx* c, int mode, bool many, cudaStream_t st, const FrameArgs& a, uint32_t pass) {
-    if (mode == 0 && many) {
-        k_shade_rows<0><<<shade_grid(c, kShadeRowsMode, false), 256, 0, st>>>(a, pass);
+static void launch_shade(const ve_ctx* c, int mode, cudaStream_t st, const FrameArgs& a, uint32_t pass) {
+    if (mode == kShadeRowsMode) {
+        k_shade_rows<0><<<shade_grid(c, mode, false), 256, 0, st>>>(a, pass);
         return;
     }
     const uint32_t grid = shade_grid(c, mode, false);
@@ -3250,20 +3245,48 @@ static int ensure_copy_stream(ve_ctx* c) {
     return VE_OK;
 }
 
-static void launch_trace(const ve_ctx* c, cudaStream_t st, const FrameArgs& a, uint32_t pass, bool count, bool em,
-                         bool flat, bool one) {
-    const uint32_t g = uint32_t(count ? c->grid_trace_count : one ? c->grid_trace_one : c->grid_trace);
+static void launch_trace(const ve_ctx* c, cudaStream_t st, const FrameArgs& a, uint32_t pass, bool em, TraceKind kind) {
+    const uint32_t g = resident_grid(c, c->launch.trace_blocks_per_sm, c->occ_trace[em][kind]);
     if (em) {
-        if (count) k_trace<true, true><<<g, 256, 0, st>>>(a, pass);
-        else if (one) k_trace<false, true, true, true><<<g, 256, 0, st>>>(a, pass);
-        else if (flat) k_trace<false, true, true><<<g, 256, 0, st>>>(a, pass);
-        else k_trace<false, true><<<g, 256, 0, st>>>(a, pass);
+        switch (kind) {
+            case kTraceCount: k_trace<true, true><<<g, 256, 0, st>>>(a, pass); break;
+            case kTraceOne: k_trace<false, true, true, true><<<g, 256, 0, st>>>(a, pass); break;
+            case kTraceFlat: k_trace<false, true, true><<<g, 256, 0, st>>>(a, pass); break;
+            default: k_trace<false, true><<<g, 256, 0, st>>>(a, pass); break;
+        }
     } else {
-        if (count) k_trace<true><<<g, 256, 0, st>>>(a, pass);
-        else if (one) k_trace<false, false, true, true><<<g, 256, 0, st>>>(a, pass);
-        else if (flat) k_trace<false, false, true><<<g, 256, 0, st>>>(a, pass);
-        else k_trace<false><<<g, 256, 0, st>>>(a, pass);
+        switch (kind) {
+            case kTraceCount: k_trace<true><<<g, 256, 0, st>>>(a, pass); break;
+            case kTraceOne: k_trace<false, false, true, true><<<g, 256, 0, st>>>(a, pass); break;
+            case kTraceFlat: k_trace<false, false, true><<<g, 256, 0, st>>>(a, pass); break;
+            default: k_trace<false><<<g, 256, 0, st>>>(a, pass); break;
+        }
     }
+}
+
+// The kernel instances that a batch runs: FLAT needs a top table that reaches
+// the leaves (depth 3..10) in every view's scene, ONE the same such scene in
+// all of them.  (The views' scene ids have been checked.)
+struct Instances {
+    bool em = false;
+    TraceKind trace = kTraceGeneral;
+    int mode = 0;   // kModeEm | kModeLb | kModeNrc
+    int shade = 0;  // the mode, or kShadeRowsMode
+};
+static Instances batch_instances(const ve_ctx* c, const ve_view* views, uint32_t nv, uint32_t flags, uint64_t paths) {
+    Instances k;
+    bool flat = true, one = true;
+    for (uint32_t i = 0; i < nv; i++) {
+        one = one && views[i].scene_id == views[0].scene_id;
+        const SceneSlot& sc = c->scenes[views[i].scene_id];
+        flat = flat && sc.top_level != 0u && sc.top_level == sc.depth;
+    }
+    k.em = (flags & VE_FRAME_EMISSIVE) != 0;
+    k.trace = (flags & VE_FRAME_COUNT_FETCH) ? kTraceCount : flat && one ? kTraceOne : flat ? kTraceFlat : kTraceGeneral;
+    const bool nrc = (flags & (VE_FRAME_LEARNED | VE_FRAME_TERMINATE_HASH | VE_FRAME_TRAIN)) != 0;
+    k.mode = (k.em ? kModeEm : 0) | ((flags & VE_FRAME_LBUFFER) ? kModeLb : 0) | (nrc ? kModeNrc : 0);
+    k.shade = k.mode == 0 && paths >= kShadeRowsPaths ? kShadeRowsMode : k.mode;
+    return k;
 }
 
 static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_outputs* outs) {
@@ -3441,15 +3464,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
     }
     // emissive lights: the scenes' registries and reservoir tables, the
     // per-path NEE records
-    // the trace's FLAT instance: every view's scene has a top table reaching
-    // its leaves (depth 3..10)
-    // ... and its one-scene form: all of them show the same scene
-    bool flat = true, one = true;
-    for (uint32_t i = 0; i < nv; i++) {
-        one = one && views[i].scene_id == views[0].scene_id;
-        const SceneSlot& sc = c->scenes[views[i].scene_id];
-        flat = flat && sc.top_level != 0u && sc.top_level == sc.depth;
-    }
+    const Instances inst = batch_instances(c, views, nv, flags, paths);
     std::vector<int> em_scenes;
     if (flags & VE_FRAME_EMISSIVE) {
         for (uint32_t i = 0; i < nv; i++) {
@@ -3574,7 +3589,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
     a.out_mapped = parity ? c->out_mapped2.p : c->out_mapped.p;
     a.out_mapped8 = parity ? c->out_m82.p : c->out_m8.p;
     a.path_rgb = (flags & VE_FRAME_PATH_RGB) ? c->path_rgb.p : nullptr;
-    a.refill = refill_of(c, flat && !count);
+    a.refill = refill_of(c, inst.trace);
     a.view_offset = 0;
     a.remaining = nullptr;
     const bool learned = nrc && (flags & VE_FRAME_LEARNED);
@@ -3619,15 +3634,12 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
     }
     a.early_ids = early;
     a.own_rays = !pipe;
-    one = one && flat;
-    if (one) {
+    if (inst.trace == kTraceOne) {
         const SceneSlot& sc = c->scenes[views[0].scene_id];
         a.one = flat_scene(sc.nodes, sc.top, sc.depth);
     }
-    const bool em = (flags & VE_FRAME_EMISSIVE) != 0;
     const bool lbm = (flags & VE_FRAME_LBUFFER) != 0;
-    const bool nrcm = (flags & (VE_FRAME_LEARNED | VE_FRAME_TERMINATE_HASH | VE_FRAME_TRAIN)) != 0;
-    const int mode = (em ? kModeEm : 0) | (lbm ? kModeLb : 0) | (nrcm ? kModeNrc : 0);
+    const int mode = inst.mode;
     // the frame's kernel sequence (no host synchronisation inside)
     // part 0: the whole frame; a pipelined frame runs as part 1 (primary and
     // trace pass 0, which read no radiance cache) and part 2 (the decay and
@@ -3677,12 +3689,12 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         if (part == 2) decay();
         for (uint32_t pass = head ? 0u : 1u; pass <= (tail ? max_b + 1u : 0u); pass++) {
             if (pass > 0) {  // pass 0 runs inside the fused primary
-                launch_shade(c, mode, paths >= kShadeRowsPaths, st, a, pass);
+                launch_shade(c, inst.shade, st, a, pass);
                 launches++;
             }
             rec();
             if (pass <= max_b) {
-                launch_trace(c, st, a, pass, count, em, flat, one);
+                launch_trace(c, st, a, pass, inst.em, inst.trace);
                 launches++;
                 trace_launches++;
             }
@@ -3757,7 +3769,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
                                      flags & (VE_FRAME_COUNT_FETCH | VE_FRAME_PATH_RGB | VE_FRAME_LEARNED |
                                               VE_FRAME_TERMINATE_HASH | VE_FRAME_TRAIN | VE_FRAME_SCHEDULED |
                                               VE_FRAME_EMISSIVE | VE_FRAME_LBUFFER | VE_FRAME_SPLIT),
-                                     paths, uint64_t(c->grid_trace), uint64_t(c->grid_trace_one), uint64_t(c->grid_shade),
+                                     paths, uint64_t(c->launch.trace_blocks_per_sm), uint64_t(c->launch.shade_blocks_per_sm),
                                      uint64_t(c->launch.refill_threshold), uint64_t(uintptr_t(nrc)),
                                      uint64_t(a.nrc_ready)};
         for (auto& d : decays) {
@@ -3767,8 +3779,8 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         }
         for (int sc : em_scenes) key.push_back((1ull << 62) | uint64_t(uint32_t(sc)));
         key.push_back((1ull << 61) | uint64_t(parity));
-        key.push_back((1ull << 59) | (uint64_t(early) << 1) | uint64_t(flat));
-        if (one) key.push_back((1ull << 58) | uint64_t(uint32_t(views[0].scene_id)));  // its pointers are captured
+        key.push_back((1ull << 59) | (uint64_t(early) << 8) | uint64_t(inst.trace));
+        if (inst.trace == kTraceOne) key.push_back((1ull << 58) | uint64_t(uint32_t(views[0].scene_id)));  // its pointers are captured
         key.push_back((1ull << 60) | (uint64_t(pipe) << 16) | (uint64_t(set) << 8) | uint64_t(part));
         ve_ctx::GraphEntry* ge = nullptr;
         for (auto& g : c->graphs)
@@ -4077,15 +4089,19 @@ int ve_ctx_create(const ve_renderer_config* cfg, ve_ctx** out) {
             return fail(VE_ERR_CUDA, "ctx_create: constant table upload failed");
         }
     }
-    int bt = 0, bt1 = 0, btc = 0, bs = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt, k_trace<false>, 256, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&btc, k_trace<true>, 256, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bs, k_shade<0>, 256, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt1, k_trace<false, false, true, true>, 256, 0);
-    x->occ_trace_one = std::max(bt1, 1);
-    x->occ_trace = std::max(bt, 1);
-    x->occ_trace_count = std::max(btc, 1);
-    x->occ_shade = std::max(bs, 1);
+    {
+        int t[2][kTraceKinds] = {};
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t[0][kTraceGeneral], k_trace<false>, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t[0][kTraceFlat], k_trace<false, false, true>, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t[0][kTraceOne], k_trace<false, false, true, true>, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t[0][kTraceCount], k_trace<true>, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t[1][kTraceGeneral], k_trace<false, true>, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t[1][kTraceFlat], k_trace<false, true, true>, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t[1][kTraceOne], k_trace<false, true, true, true>, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t[1][kTraceCount], k_trace<true, true>, 256, 0);
+        for (int e = 0; e < 2; e++)
+            for (int k = 0; k < kTraceKinds; k++) x->occ_trace[e][k] = std::max(t[e][k], 1);
+    }
     {
         int o[8] = {0};
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o[0], k_shade<0>, 256, 0);
@@ -4103,7 +4119,6 @@ int ve_ctx_create(const ve_renderer_config* cfg, ve_ctx** out) {
                                                       0);
         for (int m = 0; m < 4; m++) x->occ_emit_mode[m] = std::max(e[m], 1);
     }
-    apply_launch(x);
     int rc = 0;
     for (auto& e : x->staging_ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     if ((rc = x->counters.ensure(CNT_TOTAL)) || (rc = x->stats.ensure(ST_TOTAL)) ||
@@ -5003,7 +5018,6 @@ int ve_set_launch_config(ve_ctx* c, const ve_launch_config* cfg) {
     if (!c || !cfg) return fail(VE_ERR_INVALID, "set_launch_config: null argument");
     if (cfg->refill_threshold > 32) return fail(VE_ERR_INVALID, "set_launch_config: refill_threshold must be <= 32");
     c->launch = *cfg;
-    apply_launch(c);
     return VE_OK;
 }
 
@@ -5016,7 +5030,6 @@ int ve_autotune(ve_ctx* c, const ve_view* views, uint32_t nv, uint32_t frames, v
     for (auto& v : tv) v.frame.flags = (v.frame.flags | VE_FRAME_TIMING) & ~VE_FRAME_PATH_RGB;
     auto measure = [&](const ve_launch_config& cfg, float* ms) -> int {
         c->launch = cfg;
-        apply_launch(c);
         int rc = render_batch(c, tv.data(), nv, nullptr);  // warm-up at this shape
         if (rc) return rc;
         VE_CUDA(cudaStreamSynchronize(c->stream));
@@ -5029,19 +5042,19 @@ int ve_autotune(ve_ctx* c, const ve_view* views, uint32_t nv, uint32_t frames, v
         *ms = (c->tot_ms[0] - t0) / float(frames);
         return VE_OK;
     };
-    ve_launch_config cur{uint32_t(c->occ_trace_one), uint32_t(c->occ_shade), ve::kDefaultRefill, 0};
+    ve_launch_config cur{uint32_t(c->occ_trace[0][kTraceOne]), uint32_t(c->occ_shade_mode[0]), ve::kDefaultRefill, 0};
     float best_ms = 0.0f;
     int rc = measure(cur, &best_ms);
     if (rc) return rc;
     // coordinate descent: trace blocks/SM, shade blocks/SM, refill threshold
-    for (int tb = 1; tb <= c->occ_trace_one; tb++) {
+    for (int tb = 1; tb <= c->occ_trace[0][kTraceOne]; tb++) {
         ve_launch_config t = cur;
         t.trace_blocks_per_sm = uint32_t(tb);
         float ms = 0;
         if ((rc = measure(t, &ms))) return rc;
         if (ms < best_ms) { best_ms = ms; cur = t; }
     }
-    for (int sb = 1; sb <= c->occ_shade; sb++) {
+    for (int sb = 1; sb <= c->occ_shade_mode[0]; sb++) {
         ve_launch_config t = cur;
         t.shade_blocks_per_sm = uint32_t(sb);
         float ms = 0;
@@ -5056,7 +5069,6 @@ int ve_autotune(ve_ctx* c, const ve_view* views, uint32_t nv, uint32_t frames, v
         if (ms < best_ms) { best_ms = ms; cur = t; }
     }
     c->launch = cur;
-    apply_launch(c);
     if (best) *best = cur;
     return VE_OK;
 }

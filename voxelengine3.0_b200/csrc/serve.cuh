@@ -310,14 +310,15 @@ static void serve_loop(ve_server* s) {
             }
         }
         // 2. one shade + one trace pass over every live path
-        k_shade<0><<<c->grid_shade, 256, 0, st>>>(a, ps);
+        k_shade<0><<<shade_grid(c, 0, false), 256, 0, st>>>(a, ps);
         bool flat = true;  // every scene with paths in flight has a table reaching its leaves
         for (const ServeRequest* r : run) {
             const SceneSlot& sc = c->scenes[r->view.scene_id];
             flat = flat && sc.top_level != 0u && sc.top_level == sc.depth;
         }
-        a.refill = refill_of(c, flat);
-        launch_trace(c, st, a, ps, false, false, flat, false);
+        const TraceKind kind = flat ? kTraceFlat : kTraceGeneral;
+        a.refill = refill_of(c, kind);
+        launch_trace(c, st, a, ps, false, kind);
         if (ps == kRing - 1)  // wrap: the survivors' count moves to slot 0
             cudaMemcpyAsync(c->counters.p + CNT_LIVE, c->counters.p + CNT_LIVE + kRing, 4, cudaMemcpyDeviceToDevice,
                             st);
