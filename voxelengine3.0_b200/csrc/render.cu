@@ -5042,19 +5042,35 @@ int ve_autotune(ve_ctx* c, const ve_view* views, uint32_t nv, uint32_t frames, v
         *ms = (c->tot_ms[0] - t0) / float(frames);
         return VE_OK;
     };
-    ve_launch_config cur{uint32_t(c->occ_trace[0][kTraceOne]), uint32_t(c->occ_shade_mode[0]), ve::kDefaultRefill, 0};
+    // Every instance starts at its own occupancy maximum: the largest of any,
+    // which each grid clamps.  If that stays the best, later batches of other
+    // instances run at theirs too.
+    int occ_t = 1, occ_s = 1;
+    for (const auto& e : c->occ_trace)
+        for (int o : e) occ_t = std::max(occ_t, o);
+    for (int o : c->occ_shade_mode) occ_s = std::max(occ_s, o);
+    ve_launch_config cur{uint32_t(occ_t), uint32_t(occ_s), 0, 0};
     float best_ms = 0.0f;
     int rc = measure(cur, &best_ms);
     if (rc) return rc;
-    // coordinate descent: trace blocks/SM, shade blocks/SM, refill threshold
-    for (int tb = 1; tb <= c->occ_trace[0][kTraceOne]; tb++) {
+    uint32_t flags = 0;
+    uint64_t paths = 0;
+    for (const ve_view& v : tv) {
+        flags |= v.frame.flags;
+        paths += view_paths(v.frame);
+    }
+    const Instances inst = batch_instances(c, tv.data(), nv, flags, paths);
+    cur.refill_threshold = refill_of(c, inst.trace);  // (as measured)
+    // coordinate descent: trace blocks/SM, shade blocks/SM, refill threshold;
+    // only shapes that the views' instances can take
+    for (int tb = 1; tb < c->occ_trace[inst.em][inst.trace]; tb++) {
         ve_launch_config t = cur;
         t.trace_blocks_per_sm = uint32_t(tb);
         float ms = 0;
         if ((rc = measure(t, &ms))) return rc;
         if (ms < best_ms) { best_ms = ms; cur = t; }
     }
-    for (int sb = 1; sb <= c->occ_shade_mode[0]; sb++) {
+    for (int sb = 1; sb < c->occ_shade_mode[inst.shade]; sb++) {
         ve_launch_config t = cur;
         t.shade_blocks_per_sm = uint32_t(sb);
         float ms = 0;
@@ -5063,6 +5079,7 @@ int ve_autotune(ve_ctx* c, const ve_view* views, uint32_t nv, uint32_t frames, v
     }
     for (uint32_t thr : {4u, 8u, 12u, 16u, 20u, 24u, 28u}) {
         ve_launch_config t = cur;
+        if (thr == cur.refill_threshold) continue;
         t.refill_threshold = thr;
         float ms = 0;
         if ((rc = measure(t, &ms))) return rc;
