@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(256, 4) k_nrc_encode(Args a, uint8_t* __restri
 // a call with 262147 rows took 1.78 ms, 0.1 of it on the GPU.
 struct StoreOut {
     float* out;
-    __device__ __forceinline__ void operator()(uint8_t*, uint32_t row, bool valid, const float (&y)[3]) const {
+    __device__ __forceinline__ void operator()(uint32_t row, bool valid, const float (&y)[3]) const {
         if (!valid) return;
         out[3ull * row + 0] = y[0];
         out[3ull * row + 1] = y[1];
@@ -516,9 +516,8 @@ struct StoreOut {
 // each with its own operand tile, tensor-memory columns (M = 128
 // accumulator, lanes 0-127) and mbarrier, so one group's tile copy and
 // epilogue overlap the other's tensor-core work; three CTAs per SM (shared
-// memory, and 384 of the 512 tensor-memory columns).  `epi(scratch, row,
-// valid, y)` is called by all 128 threads of a group with the row's
-// prediction; `scratch` is 4 KB of shared memory free during the call.
+// memory, and 384 of the 512 tensor-memory columns).  `epi(row, valid, y)` is
+// called by all 128 threads of a group with the row's prediction.
 template <class Epi>
 __global__ void __launch_bounds__(256, 3) k_nrc_infer(Args a, const uint8_t* __restrict__ X, Epi epi) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -601,7 +600,7 @@ __global__ void __launch_bounds__(256, 3) k_nrc_infer(Args a, const uint8_t* __r
             }
         }
         if (timed_out) break;
-        epi(sh, row, valid, y);  // the last layer's operands are consumed: sh is scratch
+        epi(row, valid, y);
         tc::fence_before();
         group_sync(g);
     }

@@ -1438,7 +1438,6 @@ __global__ void __launch_bounds__(256, shade_ctas(MODE)) k_shade(FrameArgs a, ui
 // every warp is at the queue counters.
 constexpr uint64_t kShadeRowsPaths = 3ull << 19;  // path slots of a batch from which it is taken
 constexpr uint32_t kShadeRows = 4;                // rows of 32 paths
-template <int MODE = 0>
 __global__ void __launch_bounds__(256, 4) k_shade_rows(FrameArgs a, uint32_t pass) {
     __shared__ uint2 order[8][32 * kShadeRows];  // per warp: {live entry, view}, those that hit first
     __shared__ uint4 next[7][256];               // per thread: the state of its path in the next row
@@ -1504,8 +1503,8 @@ __global__ void __launch_bounds__(256, 4) k_shade_rows(FrameArgs a, uint32_t pas
             ps.tp = *reinterpret_cast<const float4*>(&next[5][threadIdx.x]);
             ps.ray_d = *reinterpret_cast<const float4*>(&next[6][threadIdx.x]);
             fetch(j + 32u);
-            if (j < m) shade_path<MODE>(a, p, j < n_hit, ps, o);
-            shade_finish<MODE>(a, p, o, cnt);
+            if (j < m) shade_path<0>(a, p, j < n_hit, ps, o);
+            shade_finish<0>(a, p, o, cnt);
             const unsigned l = __ballot_sync(0xffffffffu, o.app_live), x = __ballot_sync(0xffffffffu, o.app_ext),
                            h = __ballot_sync(0xffffffffu, o.app_sh);
             if (lane == c) {
@@ -1912,7 +1911,7 @@ struct StagePath {
 // k_nrc_infer, on the 128 threads of a warpgroup (warp-aggregated deposits).
 struct ApplyDeposit {
     FrameArgs a;
-    __device__ __forceinline__ void operator()(uint8_t*, uint32_t row, bool valid, const float (&y)[3]) const {
+    __device__ __forceinline__ void operator()(uint32_t row, bool valid, const float (&y)[3]) const {
         float dr = 0.0f, dg = 0.0f, db = 0.0f, dl2 = 0.0f;
         uint32_t dvid = 0, dscene = 0;
         if (valid) {
@@ -3150,7 +3149,7 @@ static uint32_t shade_grid(const ve_ctx* c, int mode, bool emit) {
 
 static void launch_shade(const ve_ctx* c, int mode, cudaStream_t st, const FrameArgs& a, uint32_t pass) {
     if (mode == kShadeRowsMode) {
-        k_shade_rows<0><<<shade_grid(c, mode, false), 256, 0, st>>>(a, pass);
+        k_shade_rows<<<shade_grid(c, mode, false), 256, 0, st>>>(a, pass);
         return;
     }
     const uint32_t grid = shade_grid(c, mode, false);
@@ -4109,7 +4108,7 @@ int ve_ctx_create(const ve_renderer_config* cfg, ve_ctx** out) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o[kModeLb], k_shade<kModeLb>, 256, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o[kModeEm | kModeLb], k_shade<kModeEm | kModeLb>, 256, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o[kModeNrc], k_shade<kModeNrc>, 256, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o[kShadeRowsMode], k_shade_rows<0>, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o[kShadeRowsMode], k_shade_rows, 256, 0);
         for (int m = 0; m < 8; m++) x->occ_shade_mode[m] = std::max(o[m], 1);
         int e[4] = {0};
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e[0], k_sched_emit<0>, 256, 0);
