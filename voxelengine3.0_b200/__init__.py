@@ -713,7 +713,8 @@ class Renderer:
         h = _P()
         _check(self._lib.ve_ctx_create(ctypes.byref(cfg), ctypes.byref(h)))
         self._h = h
-        _results.opened()
+        self._results = _results  # (close may run at the interpreter's exit, when the module is empty)
+        self._results.opened()
         self._children: List[object] = []
         self.hash_log2 = hash_log2
         self.scene: Optional[int] = None
@@ -725,7 +726,7 @@ class Renderer:
         if getattr(self, "_h", None):
             self._lib.ve_ctx_destroy(self._h)
             self._h = None
-            _results.closed()
+            self._results.closed()
 
     __del__ = close
 
