@@ -3244,6 +3244,20 @@ static int ensure_copy_stream(ve_ctx* c) {
     return VE_OK;
 }
 
+// A call's copies into the caller's arrays on a stream of their own: a return
+// before done(), on an error after they were enqueued, waits for them.
+struct CopiesInFlight {
+    cudaStream_t stream = nullptr;
+    ~CopiesInFlight() {
+        if (stream) cudaStreamSynchronize(stream);
+    }
+    cudaError_t done() {
+        cudaStream_t s = stream;
+        stream = nullptr;
+        return s ? cudaStreamSynchronize(s) : cudaSuccess;
+    }
+};
+
 static void launch_trace(const ve_ctx* c, cudaStream_t st, const FrameArgs& a, uint32_t pass, bool em, TraceKind kind) {
     const uint32_t g = resident_grid(c, c->launch.trace_blocks_per_sm, c->occ_trace[em][kind]);
     if (em) {
@@ -3818,6 +3832,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         VE_CUDA(cudaGraphLaunch(ge->exec, st));
         return VE_OK;
     };
+    CopiesInFlight id_copies;
     if (!pipe && !early) {
         if ((rc = run(0))) return rc;
     } else {
@@ -3827,6 +3842,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
         if (early && pipe) VE_CUDA(cudaStreamWaitEvent(st, c->set_cache_done[set ^ 1], 0));
         if ((rc = run(1))) return rc;
         if (early) {
+            id_copies.stream = c->copy_stream;
             VE_CUDA(cudaEventRecord(c->frame_done, st));
             VE_CUDA(cudaStreamWaitEvent(c->copy_stream, c->frame_done, 0));
             uint64_t pb = 0;
@@ -3917,7 +3933,7 @@ static int render_batch(ve_ctx* c, const ve_view* views, uint32_t nv, ve_frame_o
             qb += nq;
         }
         VE_CUDA(cudaStreamSynchronize(st));
-        if (early) VE_CUDA(cudaStreamSynchronize(c->copy_stream));
+        VE_CUDA(id_copies.done());
     }
     if (set == 1) {
         VE_CUDA(cudaEventRecord(c->alt_done, st));
@@ -4708,6 +4724,8 @@ int ve_raycast_batch(ve_ctx* c, int32_t id, const float* origins, const float* d
     if (pieces > 1)
         if (int e = ensure_copy_stream(c)) return e;
     cudaStream_t cs = pieces > 1 ? c->copy_stream : st;
+    CopiesInFlight copies;
+    copies.stream = cs;
     float* d_o = c->ray_in.p;
     float* d_d = c->ray_in.p + 3 * n;
     for (uint64_t k = 0; k < pieces; k++) {
@@ -4726,7 +4744,7 @@ int ve_raycast_batch(ve_ctx* c, int32_t id, const float* origins, const float* d
         }
         VE_CUDA(cudaMemcpyAsync(out + 8 * b, c->ray_out.p + 8 * b, 32 * m, cudaMemcpyDeviceToHost, cs));
     }
-    VE_CUDA(cudaStreamSynchronize(cs));
+    VE_CUDA(copies.done());
     return VE_OK;
 }
 
