@@ -256,9 +256,9 @@ int ve_ctx_synchronize(ve_ctx* ctx);
 /* Orders work enqueued on the context's stream after this call behind every
  * frame rendered so far (VE_CFG_PIPELINE runs some on a second stream). */
 int ve_ctx_join(ve_ctx* ctx);
-/* Pinned host memory for result arrays (any context may copy into it; a forked
- * child has its own copy; freed
- * by the caller once no copy into it is in flight). */
+/* Pinned host memory for result arrays: any context may copy into it, a forked
+ * child has its own copy, and the caller frees it once no copy into it is in
+ * flight. */
 int ve_host_alloc(uint64_t bytes, void** out);
 int ve_host_free(void* p);
 
@@ -271,7 +271,9 @@ int ve_scene_upload(ve_ctx* ctx, const uint32_t* words, uint64_t n_words, uint32
  * OctreeCPU::insert of every voxel followed by Octree::set produce, built on
  * the device from n host rows (x, y, z, material 1..127) — a repeated
  * position keeps its last row — and uploaded as a scene like
- * ve_scene_upload.  *n_words (may be NULL) receives the array size. */
+ * ve_scene_upload.  *n_words (may be NULL) receives the array size.  The
+ * context keeps up to 512 MB of the scratch of builds and normal passes for the
+ * next one; the driver takes it back when an allocation would fail. */
 int ve_scene_build(ve_ctx* ctx, const uint32_t* xyzm, uint64_t n, uint32_t depth, uint32_t flags,
                    int32_t* scene_id, uint64_t* n_words);
 int ve_scene_release(ve_ctx* ctx, int32_t scene_id);
@@ -319,7 +321,8 @@ int ve_raycast_batch(ve_ctx* ctx, int32_t scene_id, const float* origins, const 
                      uint32_t controlchecks, uint32_t flags, uint32_t* out);
 /* device bytes held by a scene: node array, radiance cache and top table
  * (4 B per cell of the grid one level above the leaves and of the layer of
- * cells at 2^D, for depths up to 10: 530 MiB at depth 10 and deeper) */
+ * cells at 2^D, for depths up to 10: 530 MiB at depth 10 and deeper), without
+ * the context's own buffers */
 int ve_scene_footprint(ve_ctx* ctx, int32_t scene_id, uint64_t* bytes);
 /* The box bounce rays are clipped to (no reference counterpart: a bound the
  * trace derives from the top table).  A bounce ray whose escape and timeout

@@ -285,13 +285,13 @@ class _ResultPool:
 
     A fresh pageable array costs its page faults and the driver's staging copy
     on every call.  A pinned one is written by the GPU directly, and is used
-    again once the program has dropped the arrays it was under: a call with 12
-    mixed views (165 MB of results) takes 5.4 ms instead of 25, 1 M rays 2.6
-    instead of 6.5, a 256x256 frame 0.17 instead of 0.41.
+    again once the program has dropped the arrays it was under: a 1080p frame's
+    ids and rgb (33 MB) take 1.1 ms instead of 5.3, 1 M rays 2.1 instead of 6, a
+    256x256 frame 0.16 instead of 0.47.
 
-    Pinning a new block costs what three to five calls then save, so a size is
-    pinned when it is asked for the second time, and its first call costs what
-    it does with ordinary arrays.  A free block serves any size from half its
+    Pinning a new block costs what two to five calls then save (1080p 5 ms,
+    853x479 3.3, 256x256 1.2), so a size is pinned when it is asked for the second
+    time, and its first call costs what it does with ordinary arrays.  A free block serves any size from half its
     own up.  At most LIMIT bytes are held, in use or not, the free blocks longest
     unused making room; beyond that, and under MIN bytes (where a pageable copy
     is as quick), results come in ordinary arrays.  The blocks not in use are

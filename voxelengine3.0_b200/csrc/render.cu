@@ -1209,9 +1209,9 @@ __device__ __forceinline__ void shade_emit(const FrameArgs& a, uint32_t p, const
 // hit in registers (the same shade_step the shade pass runs), appending its
 // rays and live entry for trace pass 0 / shade pass 1 — the frame's largest
 // shade pass never round-trips the path state through memory.
-// 4 CTAs/SM (64 registers, ~110 B of spills in the plain instance): the
+// 4 CTAs/SM (64 registers, 68 B of spill stores in the plain instance): the
 // kernel is latency-bound, and the extra warps beat the spills (0.49 -> 0.44
-// ms per 1080p depth-10 frame).
+// ms per 1080p depth-10 frame when that was tried; 0.320 since).
 template <bool COUNT, bool FUSED, int MODE = 0>
 __global__ void __launch_bounds__(256, 4) k_primary(FrameArgs a) {
     const uint32_t tile = blockIdx.x + a.tile_offset;
@@ -2354,7 +2354,10 @@ constexpr uint64_t kKeptEdits = 1u << 20;
 constexpr uint64_t kRayPiece = 1u << 17;
 
 // bytes of freed build and normal-pass scratch a context keeps for its next
-// build (the pool is emptied with the context)
+// build (the pool goes with the context; a cudaMalloc that would fail gets its
+// memory: with 40 MB of the device left, a scene of 180 MB was uploaded).  The first
+// upload of a context, whose pool is still to grow, takes 1.6 / 3.3 / 10.9 / 39.6
+// ms at depth 7 / 8 / 9 / 10, with cudaMalloc and cudaFree 2.6 / 4.9 / 11.5 / 39.7.
 constexpr uint64_t kScratchKept = 512ull << 20;
 constexpr size_t kScratchLarge = 128u << 20;  // larger pieces are allocated and freed each time
 
