@@ -127,3 +127,25 @@ def test_blocks_that_end_inside_the_pool_and_in_threads(ve, pool):
     gc.collect()
     pool.closed()
     assert pool._held == 0 and not pool._free and not pool.live
+
+
+def test_a_renderer_that_ends_inside_the_pool(ve, pool):
+    """A collection inside an allocation closes another renderer on this thread."""
+    lib = ve.load_library()
+    alloc = lib.ve_host_alloc
+    pool.opened()
+
+    def closing(size, out):
+        pool.closed()
+        return alloc(size, out)
+
+    pool.empty((MB,), np.uint8)
+    lib.ve_host_alloc = closing
+    done = []
+    t = threading.Thread(target=lambda: done.append(pool.empty((MB,), np.uint8)), daemon=True)
+    t.start()
+    t.join(20)
+    assert done and pinned(pool, done[0]) and pool._renderers == 1
+    done.clear()
+    pool.closed()
+    assert pool._renderers == 0 and not pool.live and pool._held == 0

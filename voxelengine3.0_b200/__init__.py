@@ -303,8 +303,9 @@ class _ResultPool:
 
     def __init__(self):
         self._lock = threading.Lock()
-        # blocks given back: a collection may end one anywhere, inside these
-        # methods too, so the owner only leaves it here for whoever has the lock
+        # blocks given back and renderers closed (None): a collection may end
+        # either anywhere, inside these methods too, so they are only left here
+        # for whoever has the lock
         self._returned: collections.deque = collections.deque()
         self._free: Dict[int, List[tuple]] = {}  # size -> (time given back, address), oldest first
         self._asked: set = set()  # sizes asked for before
@@ -364,7 +365,7 @@ class _ResultPool:
         self._settle()
 
     def _settle(self) -> None:
-        """Files the blocks given back, unless who has the lock will do it."""
+        """Files what was left, unless who has the lock will do it."""
         while self._returned and self._lock.acquire(blocking=False):
             try:
                 self._collect()
@@ -373,10 +374,14 @@ class _ResultPool:
 
     def _collect(self) -> None:
         while self._returned:
-            ptr, size = self._returned.popleft()
+            block = self._returned.popleft()
+            if block is None:
+                self._renderers -= 1
+                continue
             self._time += 1
-            self._free.setdefault(size, []).append((self._time, ptr))
+            self._free.setdefault(block[1], []).append((self._time, block[0]))
         if self._renderers == 0:
+            self._asked.clear()
             self._trim()
 
     def _release(self, size: int) -> None:
@@ -395,11 +400,7 @@ class _ResultPool:
             self._renderers += 1
 
     def closed(self) -> None:
-        with self._lock:
-            self._renderers -= 1
-            if self._renderers == 0:
-                self._asked.clear()
-            self._collect()
+        self._returned.append(None)
         self._settle()
 
 
