@@ -437,11 +437,14 @@ int ve_server_submit(ve_server* s, const ve_view* v, uint32_t* voxel_id_out, flo
     cudaSetDevice(s->c->device);
     cudaEventCreateWithFlags(&r->done_ev, cudaEventDisableTiming);
     {
-        std::lock_guard<std::mutex> lk(s->mu);
+        std::unique_lock<std::mutex> lk(s->mu);
         if (s->stop) {
+            const int code = s->error ? s->error : VE_ERR_STATE;
+            const std::string msg = s->error_msg;
+            lk.unlock();  // (as in ve_server_wait)
             cudaEventDestroy(r->done_ev);
             delete r;
-            return fail(s->error ? s->error : VE_ERR_STATE, "server_submit: server stopped: " + s->error_msg);
+            return fail(code, "server_submit: server stopped: " + msg);
         }
         r->id = s->next_id++;
         r->t_submit = now_s();
@@ -472,8 +475,12 @@ int ve_server_wait(ve_server* s, uint64_t id, uint32_t timeout_ms, ve_request_in
         info->pixels = r->pixels;
         info->paths = r->paths;
     }
-    cudaEventDestroy(r->done_ev);
     s->all.erase(it);
+    // no CUDA call under the lock: the worker may be inside one (the copy of a
+    // later request into pageable memory) that waits for serve_copied of an
+    // earlier request, which takes the lock
+    lk.unlock();
+    cudaEventDestroy(r->done_ev);
     delete r;
     return VE_OK;
 }
