@@ -3280,9 +3280,11 @@ static void launch_trace(const ve_ctx* c, cudaStream_t st, const FrameArgs& a, u
     }
 }
 
-// The kernel instances that a batch runs: FLAT needs a top table that reaches
-// the leaves (depth 3..10) in every view's scene, ONE the same such scene in
-// all of them.  (The views' scene ids have been checked.)
+// The scene's top table reaches its leaves (depth 3..10).
+static bool flat_table(const SceneSlot& sc) { return sc.top_level != 0u && sc.top_level == sc.depth; }
+
+// The kernel instances that a batch runs: FLAT needs such a table in every
+// view's scene, ONE the same such scene in all of them.  (The views' scene ids have been checked.)
 struct Instances {
     bool em = false;
     TraceKind trace = kTraceGeneral;
@@ -3294,8 +3296,7 @@ static Instances batch_instances(const ve_ctx* c, const ve_view* views, uint32_t
     bool flat = true, one = true;
     for (uint32_t i = 0; i < nv; i++) {
         one = one && views[i].scene_id == views[0].scene_id;
-        const SceneSlot& sc = c->scenes[views[i].scene_id];
-        flat = flat && sc.top_level != 0u && sc.top_level == sc.depth;
+        flat = flat && flat_table(c->scenes[views[i].scene_id]);
     }
     k.em = (flags & VE_FRAME_EMISSIVE) != 0;
     k.trace = (flags & VE_FRAME_COUNT_FETCH) ? kTraceCount : flat && one ? kTraceOne : flat ? kTraceFlat : kTraceGeneral;

@@ -85,6 +85,8 @@ struct ServeRequest {
     uint32_t* out_vid = nullptr;
     float* out_rgb = nullptr;
     int state = 0;  // 0 queued, 1 on the GPU, 2 resolving, 3 done, 4 failed
+    bool flat = false;  // its scene's table reaches the leaves (told at submission: the
+                        // worker reads no host scene, whose table other calls extend)
     uint32_t slot = 0;
     uint64_t pix_off = 0, path_off = 0, pixels = 0, paths = 0;
     uint32_t tiles = 0;
@@ -312,10 +314,7 @@ static void serve_loop(ve_server* s) {
         // 2. one shade + one trace pass over every live path
         k_shade<0><<<shade_grid(c, 0, false), 256, 0, st>>>(a, ps);
         bool flat = true;  // every scene with paths in flight has a table reaching its leaves
-        for (const ServeRequest* r : run) {
-            const SceneSlot& sc = c->scenes[r->view.scene_id];
-            flat = flat && sc.top_level != 0u && sc.top_level == sc.depth;
-        }
+        for (const ServeRequest* r : run) flat = flat && r->flat;
         const TraceKind kind = flat ? kTraceFlat : kTraceGeneral;
         a.refill = refill_of(c, kind);
         launch_trace(c, st, a, ps, false, kind);
@@ -425,6 +424,7 @@ int ve_server_submit(ve_server* s, const ve_view* v, uint32_t* voxel_id_out, flo
     ServeRequest* r = new ServeRequest();
     r->owner = s;
     r->view = *v;
+    r->flat = flat_table(s->c->scenes[v->scene_id]);
     r->out_vid = voxel_id_out;
     r->out_rgb = rgb_out;
     r->pixels = uint64_t(f.width) * f.height;
