@@ -4716,6 +4716,7 @@ int ve_raycast_batch(ve_ctx* c, int32_t id, const float* origins, const float* d
     if (!origins || !dirs || !out) return fail(VE_ERR_INVALID, "raycast_batch: null argument");
     if (n > (1ull << 28)) return fail(VE_ERR_CAPACITY, "raycast_batch: at most 2^28 rays per call");
     if (controlchecks > kMaxControlChecks) return fail(VE_ERR_INVALID, "raycast_batch: controlchecks must be <= 65536");
+    cudaSetDevice(c->device);  // the buffers and the copy stream are made on it
     int rc;
     if ((rc = c->ray_in.ensure(6 * n)) || (rc = c->ray_out.ensure(8 * n))) return rc;
     const SceneSlot& sl = c->scenes[id];
